@@ -16,8 +16,15 @@
 //      EPI_TOPK: the k best (distance, index) pairs, one per lane, kept
 //        sorted by warp ballots (ties broken by the smaller index, self
 //        excluded) -- the exact kNN, unique under that total order;
-//      EPI_RANK: per lane m < k, the number of points strictly better than
-//        threshold m -- the ranks trustworthiness needs.
+//      EPI_RANK: per threshold m < k, the number of points strictly better
+//        than it -- the ranks trustworthiness needs. A query's thresholds are
+//        sorted once into shared memory; a point within the largest finds the
+//        first threshold it is better than by binary search and adds one to
+//        that threshold's count, and the counts' prefix sums are the answer.
+//        (Comparing every point with every threshold by shuffles took five
+//        times as long as the distances themselves: trustworthiness and
+//        preservation of 10k queries x 100k points x 50 dims, k = 15, whole
+//        call: 43.2 ms then, 18.4 ms with the search.)
 //    Few queries (the metrics' subsample) split the point range into slices
 //    (partial lists merged by k_knn_merge, rank counts added atomically).
 //  * trustworthiness (sklearn.manifold.trustworthiness's definition) over a
@@ -44,10 +51,16 @@ constexpr unsigned kFull = 0xffffffffu;
 
 enum { EPI_TOPK = 0, EPI_RANK = 1 };
 
+template <int EPI>
 struct __align__(16) TileSmem {
     float q[2][kDC][kQS];
     float p[2][kDC][kPS];
     uint32_t qrow[kQT];
+    // EPI_RANK: each query's thresholds ascending, which of the given ones
+    // each is, and the points counted per sorted threshold
+    float thr[EPI == EPI_RANK ? kQT : 1][32];
+    uint32_t hist[EPI == EPI_RANK ? kQT : 1][32];
+    uint8_t given[EPI == EPI_RANK ? kQT : 1][32];
 };
 
 __device__ __forceinline__ void cp_async4(float *smem, const float *gmem, bool ok)
@@ -138,7 +151,7 @@ __device__ __forceinline__ void list_offer(float &ld, uint32_t &li, const float 
 template <bool EUC, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
 {
-    __shared__ TileSmem S;
+    __shared__ TileSmem<EPI> S;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q0 = blockIdx.x * kQT;
     const uint32_t slice = blockIdx.y;
@@ -155,9 +168,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
     // per-query state of this warp's 8 queries
     float ld[8];
     uint32_t li[8];
-    uint32_t cnt[8];
-    float td[8];
-    uint32_t tj[8];
+    float thmax[8];      // EPI_RANK: the query's largest threshold
+    uint32_t n_thr[8];   // EPI_RANK: thresholds that are numbers (no point is better than a NaN)
+    uint32_t place[8];   // EPI_RANK: place of threshold `lane` among the sorted ones (~0: NaN)
     uint32_t gq[8];
     bool qok[8];
 #pragma unroll
@@ -167,12 +180,32 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
         gq[i] = S.qrow[ql];
         ld[i] = __int_as_float(0x7f800000);
         li[i] = ~0u;
-        cnt[i] = 0;
-        td[i] = 0.0f;
-        tj[i] = 0;
-        if (EPI == EPI_RANK && qok[i] && lane < A.k) {
-            td[i] = A.thr_d[(size_t)(q0 + ql) * A.k + lane];
-            tj[i] = A.thr_j[(size_t)(q0 + ql) * A.k + lane];
+        thmax[i] = 0.0f;
+        n_thr[i] = 0;
+        place[i] = ~0u;
+        if (EPI == EPI_RANK && qok[i]) {  // warp-uniform
+            float td = __int_as_float(0x7fffffff);
+            uint32_t tj = ~0u;
+            if (lane < A.k) {
+                td = A.thr_d[(size_t)(q0 + ql) * A.k + lane];
+                tj = A.thr_j[(size_t)(q0 + ql) * A.k + lane];
+            }
+            uint32_t at = 0;  // a repeated neighbour keeps the order of the lanes
+            for (uint32_t m = 0; m < A.k; m++) {
+                const float od = __shfl_sync(kFull, td, m);
+                const uint32_t oj = __shfl_sync(kFull, tj, m);
+                at += (better(od, oj, td, tj) || (od == td && oj == tj && m < lane)) ? 1u : 0u;
+            }
+            S.hist[ql][lane] = 0;
+            const bool number = td == td;
+            n_thr[i] = __popc(__ballot_sync(kFull, number));
+            if (number) {
+                place[i] = at;
+                S.thr[ql][at] = td;
+                S.given[ql][at] = (uint8_t)lane;
+            }
+            __syncwarp();
+            if (n_thr[i]) thmax[i] = S.thr[ql][n_thr[i] - 1];
         }
     }
 
@@ -211,8 +244,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
             cp_async_wait<0>();
         }
         __syncthreads();
+        // dimensions past the last (staged as zeros, which change no sum) are
+        // left out in groups of four: 2 dims take 4 of the 16 steps, 50 take 52 of 64
+        const uint32_t d_left = A.dim - c * kDC;
 #pragma unroll
         for (int dd = 0; dd < kDC; dd++) {
+            if ((dd & 3) == 0 && dd && (uint32_t)dd >= d_left) break;
             const float4 qa = *reinterpret_cast<const float4 *>(&S.q[b][dd][warp * 8]);
             const float4 qb = *reinterpret_cast<const float4 *>(&S.q[b][dd][warp * 8 + 4]);
             const float4 pv = *reinterpret_cast<const float4 *>(&S.p[b][dd][lane * 4]);
@@ -253,30 +290,45 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
                     if (pidx[j] < A.n && pidx[j] != gq[i] && better(dv[j], pidx[j], thd, thi)) pend |= 1u << j;
                 list_offer<4>(ld[i], li[i], dv, pidx, pend, A.k, lane);
             } else {
-                uint32_t c_i = 0;
-                for (int src = 0; src < 32; src++) {
+                const uint32_t ql = warp * 8 + i;
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float d = __shfl_sync(kFull, dv[j], src);
-                        const uint32_t p = p0 + src * 4 + j;
-                        c_i += (p < A.n && p != gq[i] && better(d, p, td[i], tj[i])) ? 1u : 0u;
+                for (int j = 0; j < 4; j++) {
+                    if (!n_thr[i] || !(dv[j] <= thmax[i]) || pidx[j] >= A.n || pidx[j] == gq[i]) continue;
+                    // the first threshold the point is better than
+                    uint32_t lo = 0, hi = n_thr[i];
+                    while (lo < hi) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        const float t = S.thr[ql][mid];
+                        const bool before = dv[j] < t || (dv[j] == t && pidx[j] < A.thr_j[(size_t)(q0 + ql) * A.k + S.given[ql][mid]]);
+                        if (before) hi = mid;
+                        else lo = mid + 1;
                     }
+                    if (lo < n_thr[i]) atomicAdd(&S.hist[ql][lo], 1u);
                 }
-                cnt[i] += c_i;
             }
         }
     }
 
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        if (!qok[i] || lane >= A.k) continue;
+        if (!qok[i]) continue;  // warp-uniform
         const size_t q = q0 + warp * 8 + i;
         if (EPI == EPI_TOPK) {
+            if (lane >= A.k) continue;
             const size_t o = ((size_t)slice * A.nq + q) * A.k + lane;
             A.out_idx[o] = li[i];
             A.out_dist[o] = ld[i];
-        } else if (cnt[i]) {
-            atomicAdd(&A.counts[q * A.k + lane], cnt[i]);
+        } else {
+            // a point counted at a threshold is better than every later one too
+            __syncwarp();
+            uint32_t c = S.hist[warp * 8 + i][lane];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t u = __shfl_up_sync(kFull, c, off);
+                if ((int)lane >= off) c += u;
+            }
+            const uint32_t mine = __shfl_sync(kFull, c, place[i] & 31u);
+            if (lane < A.k && place[i] != ~0u && mine) atomicAdd(&A.counts[q * A.k + lane], mine);
         }
     }
 }

@@ -93,3 +93,16 @@ def test_fuzzy_cross_entropy_matches_f64_reference():
     got = umapcu.fuzzy_cross_entropy(coo, Y, a, b)
     want = fuzzy_cross_entropy(g["row"], g["col"], g["val"], Y, a, b)
     assert got == pytest.approx(want, rel=1e-10)
+
+
+@pytest.mark.parametrize("n,dim,k,metric", [(131, 3, 1, "euclidean"), (257, 17, 32, "euclidean"),
+                                            (700, 4, 31, "cosine"), (2000, 50, 15, "euclidean")])
+def test_trust_counts_with_ties(n, dim, k, metric):
+    """Ranks where points tie with the thresholds (every other point is
+    doubled; distances of a coarse grid repeat) and at the smallest and
+    largest k: sums of integers, equal to the oracle's exactly."""
+    X = np.round(_data(n, dim, n) * 2.0).astype(np.float32) + 1.0
+    X[1::2] = X[0:n - n % 2:2]
+    Y = np.random.default_rng(n).normal(size=(n, 2)).astype(np.float32)
+    q = umapcu.embedding_quality(X, Y, None, k, dist_metric=metric)
+    assert q["trust"] == O.trustworthiness(X, Y, k, metric=umapcu._metric(metric))
