@@ -30,12 +30,16 @@
 //  * trustworthiness (sklearn.manifold.trustworthiness's definition) over a
 //    query subsample, kNN preservation, fuzzy cross-entropy (f64).
 //
-// This is CUDA-core (FP32 FMA) work on purpose: the tensor-core expansion
-// |q|^2 + |p|^2 - 2 q.p changes distances in their last bits and with them
-// near-tied neighbour sets; the exact path stays bit-reproducible.
+// The distances themselves stay on the FP32 cores: the tensor-core expansion
+// |q|^2 + |p|^2 - 2 q.p changes them in their last bits and with them near-tied
+// neighbour sets. Searches of some size use the tensor cores as a filter in
+// front of them instead (knn_filter.cu), which leaves the few candidates that
+// the exact chain then orders; k_knn_tile takes the small searches, those of
+// more than 191 dims and what the filter could not settle.
 #include <cfloat>
 
 #include "internal.cuh"
+#include "knn_filter.cuh"
 
 namespace umapcu {
 namespace {
@@ -86,6 +90,8 @@ struct TileArgs {
     uint32_t n, dim, k;
     const uint32_t *qidx;    // [nq] query rows, nullptr: query q is row q
     uint32_t nq;
+    // when set: only the queries left[0 .. *n_left) (positions below nq)
+    const uint32_t *left, *n_left;
     uint32_t tiles_per_slice;
     // EPI_TOPK
     uint32_t *out_idx;       // [slices][nq][k]
@@ -154,14 +160,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
     __shared__ TileSmem<EPI> S;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q0 = blockIdx.x * kQT;
+    const uint32_t nq = A.n_left ? *A.n_left : A.nq;
+    if (q0 >= nq) return;
     const uint32_t slice = blockIdx.y;
     const uint32_t n_tiles = (A.n + kPT - 1) / kPT;
     const uint32_t t_beg = slice * A.tiles_per_slice;
     const uint32_t t_end = min(n_tiles, t_beg + A.tiles_per_slice);
     const uint32_t n_chunks = (A.dim + kDC - 1) / kDC;
     if (tid < kQT) {
-        const uint32_t q = q0 + tid;
-        S.qrow[tid] = q < A.nq ? (A.qidx ? A.qidx[q] : q) : 0u;
+        const uint32_t q = q0 + tid < nq ? (A.left ? A.left[q0 + tid] : q0 + tid) : 0u;
+        S.qrow[tid] = q0 + tid < nq ? (A.qidx ? A.qidx[q] : q) : 0u;
     }
     __syncthreads();
 
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const uint32_t ql = warp * 8 + i;
-        qok[i] = q0 + ql < A.nq;
+        qok[i] = q0 + ql < nq;
         gq[i] = S.qrow[ql];
         ld[i] = __int_as_float(0x7f800000);
         li[i] = ~0u;
@@ -219,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
         }
         for (uint32_t e = tid; e < kQT * kDC; e += kThreads) {
             const uint32_t r = e / kDC, dd = e % kDC, gd = d0 + dd;
-            const bool ok = q0 + r < A.nq && gd < A.dim;
+            const bool ok = q0 + r < nq && gd < A.dim;
             cp_async4(&S.q[b][dd][r], ok ? A.x + (size_t)S.qrow[r] * A.dim + gd : A.x, ok);
         }
         cp_async_commit();
@@ -315,7 +323,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
         const size_t q = q0 + warp * 8 + i;
         if (EPI == EPI_TOPK) {
             if (lane >= A.k) continue;
-            const size_t o = ((size_t)slice * A.nq + q) * A.k + lane;
+            // one slice writes the final place, several the merge's input
+            const size_t at = A.left && gridDim.y == 1 ? A.left[q] : q;
+            const size_t o = ((size_t)slice * A.nq + at) * A.k + lane;
             A.out_idx[o] = li[i];
             A.out_dist[o] = ld[i];
         } else {
@@ -333,13 +343,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
     }
 }
 
-// Merges the slices' partial lists: one warp per query.
+// Merges the slices' partial lists: one warp per query (left / n_left: as in
+// TileArgs).
 __global__ void k_knn_merge(const uint32_t *__restrict__ pidx, const float *__restrict__ pdist, uint32_t slices,
-                            uint32_t nq, uint32_t k, uint32_t *__restrict__ out_idx, float *__restrict__ out_dist)
+                            uint32_t nq, uint32_t k, const uint32_t *__restrict__ left,
+                            const uint32_t *__restrict__ n_left, uint32_t *__restrict__ out_idx,
+                            float *__restrict__ out_dist)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (q >= nq) return;  // warp-uniform
+    if (q >= (n_left ? *n_left : nq)) return;  // warp-uniform
     float ld = __int_as_float(0x7f800000);
     uint32_t li = ~0u;
     for (uint32_t s = 0; s < slices; s++) {
@@ -352,8 +365,9 @@ __global__ void k_knn_merge(const uint32_t *__restrict__ pidx, const float *__re
         list_offer<1>(ld, li, cd, ci, pend, k, lane);
     }
     if (lane < k) {
-        out_idx[(size_t)q * k + lane] = li;
-        out_dist[(size_t)q * k + lane] = ld;
+        const size_t at = left ? left[q] : q;
+        out_idx[at * k + lane] = li;
+        out_dist[at * k + lane] = ld;
     }
 }
 
@@ -467,6 +481,19 @@ void knn_dev(const float *d_x, uint32_t n, uint32_t dim, const uint32_t *d_qidx,
     }
     const uint32_t S = slices_for(nq, n), n_tiles = ceil_div(n, kPT);
     TileArgs A{};
+    // the tensor-core filter where it pays; the tile kernel then takes the
+    // queries it leaves (none on ordinary data)
+    DevBuf<uint32_t> left, n_left;
+    if (knn_filter_takes(n, dim, nq, k)) {
+        left.alloc(nq, s);
+        n_left.alloc(1, s);
+        check_cuda(cudaMemsetAsync(n_left.p, 0, sizeof(uint32_t), s), "memset");
+        const KnnFilterArgs F{x, n, dim, k, metric == UMAPCU_METRIC_EUCLIDEAN_SQ, d_qidx, nq, d_idx, d_dist};
+        if (knn_filter(F, left.p, n_left.p, s)) {
+            A.left = left.p;
+            A.n_left = n_left.p;
+        }
+    }
     A.x = x;
     A.n = n;
     A.dim = dim;
@@ -491,7 +518,8 @@ void knn_dev(const float *d_x, uint32_t n, uint32_t dim, const uint32_t *d_qidx,
     else k_knn_tile<false, EPI_TOPK><<<grid, kThreads, 0, s>>>(A);
     check_launch("k_knn_tile");
     if (S_eff > 1) {
-        k_knn_merge<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(pidx.p, pdist.p, S_eff, nq, k, d_idx, d_dist);
+        k_knn_merge<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(pidx.p, pdist.p, S_eff, nq, k, A.left, A.n_left,
+                                                                       d_idx, d_dist);
         check_launch("k_knn_merge");
     }
 }

@@ -1,0 +1,825 @@
+// Exact kNN by a tensor-core filter and an exact second look.
+//
+// The k nearest rows of a query are defined by the f32 FMA-chain distances of
+// knn.cu's tile kernel; computing all n of them per query is FP32 issue work
+// (166 ms for 200k x 30 dims). Here every pair is first scored on the tensor
+// cores with an error bound, and only the few points whose score could still
+// make them one of the k nearest get the exact chain:
+//
+//   score s(q, p) = q.p - |p|^2 / 2   (Euclidean; |q - p|^2 = |q|^2 - 2 s),
+//                   q.p               (cosine, unit rows),
+//
+// formed as one bf16 contraction with f32 accumulators in TMEM: a coordinate
+// is split into two bf16 pieces (hi, lo; products hi.hi, hi.lo, lo.hi) or, up
+// to kFineDim dims, three (six products, f32 accuracy), and -|p|^2 / 2 rides
+// along as three more columns against ones. Coordinates are taken relative to
+// a mean of sampled rows, which changes no difference and keeps norms small.
+//
+//   1. k_filter<.., 1> over a sample of the point tiles: per query the largest
+//      score in each of 64 groups of points. The (k + 1)-th largest of these
+//      maxima belongs to k + 1 different points, so with the error bound it
+//      gives a distance that at least k points other than the query keep to.
+//   2. k_filter_threshold turns it into the least score a true neighbour can
+//      have (bounds below).
+//   3. k_filter<.., 2> over all tiles: indices of points at or above it, about
+//      kHitTarget per query.
+//   4. k_refine: exact chain distances of those, the k best by (distance,
+//      index).
+//
+// The sample keeps step 1 at a fraction of step 3; the group maxima cost one
+// three-input maximum per two scores with no branch, step 3 the same and a
+// rarely taken branch. What bounds k_filter is the issue of its MMAs: 1.5 us a
+// 256 x 256 tile at 30 dims (6 steps of 16 columns, 0.81 us at the tensor
+// cores' rate), the same without the epilogue's arithmetic and without the
+// staging; two epilogue warps a scheduler instead of four, descriptors formed
+// in the loop and one lane issuing took 2.4 us. Against the FP32 tile kernel,
+// whole knn_exact calls: 10k x 50 dims, k = 15 1.81 -> 0.71 ms, 200k x 30 dims,
+// k = 30 166 -> 20.8 ms (of which the copies of host arrays take about 10).
+//
+// Error bound. With u = |q|, v = |p|: the split leaves at most
+// 3.1 * 2^-16 u v (two pieces) or 2^-21 u v (six products) of a dot product,
+// f32 accumulation over at most 36 steps of 16 products 1e-5 (u v + v^2 / 2),
+// centring and norms a few 2^-24 of (u + v)^2; in all |s - s_true| <=
+// kappa (u^2 + v^2) with kappa as in filter_kappa, which is rounded up. The
+// chain distance itself is within (dim + 8) 2^-24 of the true one,
+// relatively. k_filter_threshold carries both, so no true neighbour is left
+// out; a looser threshold only means more candidates.
+#include <cuda_bf16.h>
+
+#include <cfloat>
+
+#include "internal.cuh"
+#include "knn_filter.cuh"
+
+namespace umapcu {
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr uint32_t kTileN = 256;       // points per tile (the MMA's N)
+constexpr uint32_t kBlkM = 128;        // queries per accumulator (the MMA's M)
+constexpr uint32_t kChunkK = 64;       // bf16 columns per staged chunk: a 128-byte row
+constexpr uint32_t kABytes = kBlkM * kChunkK * 2;
+constexpr uint32_t kBBytes = kTileN * kChunkK * 2;
+constexpr uint32_t kGroups = 64;
+constexpr uint32_t kFineDim = 10;      // 6 dim + 3 columns still fit one chunk
+constexpr uint32_t kMaxChunks = 9;     // 144 KB of A beside two 32 KB stages of B
+constexpr uint32_t kSmemMax = 232448 - 1024;
+constexpr uint32_t kHalf = kTileN / 2; // columns of an accumulator an epilogue warp reads
+constexpr int kFilterThreads = 576;    // 16 epilogue warps, a producer, an MMA issuer
+// Candidates per query the sample is chosen for (fewer lengthen step 1, more
+// steps 3 and 4: 73 and 146 are within 3 % of each other at 200k x 30 dims),
+// and a query's list length.
+constexpr uint32_t kHitTarget = 100, kListCap = 640;
+
+struct Pack {
+    uint32_t terms, cols, steps, chunks;
+};
+
+Pack pack_of(uint32_t dim)
+{
+    Pack p;
+    p.terms = dim <= kFineDim ? 6 : 3;
+    p.cols = p.terms * dim + 3;
+    p.steps = (p.cols + 15) / 16;
+    p.chunks = (p.cols + kChunkK - 1) / kChunkK;
+    return p;
+}
+
+double filter_kappa(uint32_t terms) { return terms == 6 ? 4e-6 : 5e-5; }
+
+// ------------------------------------------------------------ preparation
+
+// Column means of up to 1024 rows spread over the data, eight columns a block:
+// any point near the data's centre serves.
+__global__ void __launch_bounds__(1024) k_filter_centre(const float *__restrict__ x, uint32_t n, uint32_t dim,
+                                                        float *__restrict__ mu)
+{
+    __shared__ float sh[128][8];
+    const uint32_t rows = min(n, 1024u), e = threadIdx.x & 7, g = threadIdx.x >> 3, d = blockIdx.x * 8 + e;
+    float acc = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t r = g + 128 * i;
+        if (r < rows && d < dim) acc += x[(size_t)((uint64_t)r * n / rows) * dim + d] / (float)rows;
+    }
+    sh[g][e] = acc;
+    __syncthreads();
+    for (uint32_t w = 64; w > 0; w >>= 1) {
+        if (g < w) sh[g][e] += sh[g + w][e];
+        __syncthreads();
+    }
+    if (g == 0 && d < dim) mu[d] = sh[0][e];
+}
+
+// |row - mu|^2 of every point, a warp per row; *bad set when a row is not
+// finite or its norm is beyond what the bound's arithmetic can hold.
+__global__ void k_filter_norms(const float *__restrict__ x, uint32_t n, uint32_t dim, const float *__restrict__ mu,
+                               float *__restrict__ norm, uint32_t *__restrict__ bad)
+{
+    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= n) return;
+    double acc = 0.0;
+    for (uint32_t d = lane; d < dim; d += 32) {
+        const double v = (double)(x[(size_t)row * dim + d] - (mu ? mu[d] : 0.0f));
+        acc += v * v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(kFull, acc, o);
+    if (lane == 0) {
+        norm[row] = (float)acc;
+        if (!(acc < 1e28)) *bad = 1u;
+    }
+}
+
+__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+// Piece t of v: what the t pieces before it leave, rounded to bf16.
+__device__ __forceinline__ float bf16_piece(float v, uint32_t t)
+{
+    float p = bf16_round(v);
+    for (uint32_t i = 0; i < t; i++) {
+        v = v - p;
+        p = bf16_round(v);
+    }
+    return p;
+}
+
+// The operands as the shared-memory images the MMA reads: K-major rows of 64
+// columns (128 bytes) in the 128-byte swizzle (16-byte unit j of row r stands
+// at j ^ (r & 7)), so that a plain bulk copy stages a chunk. Queries: blocks
+// of 128 rows, [block][chunk][128 rows]; points: tiles of 256 rows,
+// [tile][chunk][256 rows]. A thread writes one 16-byte unit (8 columns).
+// Rows past the end are zero, past the points with a score of -1e30.
+template <bool QUERY>
+__global__ void k_filter_pack(const float *__restrict__ x, uint32_t n, uint32_t dim, const float *__restrict__ mu,
+                              const float *__restrict__ norm, const uint32_t *__restrict__ qidx, uint32_t q0,
+                              uint32_t rows, uint32_t rows_pad, uint32_t terms, uint32_t chunks, bool euc,
+                              uint4 *__restrict__ out)
+{
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t units = chunks * 8;
+    if (t >= (uint64_t)rows_pad * units) return;
+    const uint32_t r = (uint32_t)(t / units), u = (uint32_t)(t % units);
+    const bool in = r < rows;
+    const uint32_t row = !in ? 0u : QUERY ? (qidx ? qidx[q0 + r] : q0 + r) : r;
+    const uint32_t cols = terms * dim;
+    __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t c = u * 8 + i;
+        float f = 0.0f;
+        if (c < cols) {
+            if (in) {
+                const uint32_t term = c / dim, d = c - term * dim;
+                // products of pieces, query x point: 00 01 10 (11 02 20)
+                const uint32_t piece = ((QUERY ? 0x201100u : 0x021010u) >> (4 * term)) & 15u;
+                const float xv = x[(size_t)row * dim + d] - (mu ? mu[d] : 0.0f);
+                f = bf16_piece(xv, piece);
+            }
+        } else if (c < cols + 3) {
+            if (QUERY) f = 1.0f;
+            else if (!in) f = c == cols ? -1e30f : 0.0f;
+            else if (euc) f = -bf16_piece(0.5f * norm[row], c - cols);
+        }
+        v[i] = __float2bfloat16_rn(f);
+    }
+    const uint32_t per = QUERY ? kBlkM : kTileN;
+    const uint32_t blk = r / per, rr = r % per, chunk = u >> 3, j = u & 7;
+    out[(((size_t)blk * chunks + chunk) * per + rr) * 8 + (j ^ (rr & 7))] = *reinterpret_cast<const uint4 *>(v);
+}
+
+// ------------------------------------------------------- PTX of the kernel
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void bar_init(uint64_t *b, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t *b, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t *b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint64_t *b, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait: false after about two seconds of clock cycles, or when another
+// role of the block has given up.
+__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile uint32_t *stop)
+{
+    if (bar_try(b, parity)) return true;
+    const long long t0 = clock64();
+    while (!bar_try(b, parity)) {
+        if (*stop) return false;
+        if (clock64() - t0 > 4000000000ll) {
+            *stop = 1u;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(b))
+                 : "memory");
+}
+// K-major, 128-byte swizzle, groups of 8 rows 1024 bytes apart
+__device__ __forceinline__ uint64_t mma_desc(uint32_t addr)
+{
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// One lane issues; the whole warp runs the loop around it, which keeps the
+// operands in uniform registers.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t *b)
+{
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(b))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+          "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+          "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(addr)
+        : "memory");
+}
+// The loaded registers are named so that no use of them moves before the wait.
+template <int N>
+__device__ __forceinline__ void tmem_wait(float (&v)[N])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < N; i++) asm volatile("" : "+f"(v[i]));
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// -------------------------------------------------------------- the filter
+
+struct FilterArgs {
+    const uint4 *a, *b;      // operand images of the query batch and the points
+    uint32_t nq, n_tiles, stride, slices;
+    uint32_t chunks, steps, stages;
+    // PASS 1
+    float *gmax;             // [parts][nq][kGroups]
+    // PASS 2
+    const float *least;      // [nq]
+    uint32_t *list;          // [parts][nq][cap]
+    uint32_t *count;         // [parts][nq], may exceed cap
+    uint32_t cap;
+    uint32_t *bad;           // set when a wait gave up
+};
+
+// One block: MB x 128 queries against the tiles slice, slice + slices, ... (of
+// every stride-th tile). Warp 16 stages point chunks through a ring of 32 KB
+// bulk copies, warp 17 issues the MMAs (128 x 256 x 16), warps 0-7 and 8-15
+// read accumulators 0 and 1 (a thread 128 columns of one query's row, in two
+// loads of 64, after which the accumulator is free). MB = 2: accumulator b holds query block b, so that one
+// is contracted while the other is read and a staged tile serves 256 queries
+// (32 bytes of L2 reads a clock where 64 would be needed with one block).
+// MB = 1, for operands of more than three chunks, whose A would not leave room
+// for the ring: the accumulators alternate between tiles. 512 columns of TMEM
+// and more than half the shared memory: one block an SM.
+template <int MB, int PASS>
+__global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P)
+{
+    extern __shared__ uint8_t dyn[];
+    __shared__ uint64_t full[8], empty[8], tfull[2], tempty[2], afull, done;
+    __shared__ uint32_t tmem_base;
+    __shared__ uint32_t stop_word;
+    volatile uint32_t *stop = &stop_word;
+    uint8_t *sa = reinterpret_cast<uint8_t *>(((uintptr_t)dyn + 1023) & ~(uintptr_t)1023);
+    uint8_t *sb = sa + (size_t)MB * P.chunks * kABytes;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t slice = blockIdx.y;
+    const uint32_t sampled = (P.n_tiles + P.stride - 1) / P.stride;
+    const uint32_t n_items = sampled > slice ? (sampled - slice + P.slices - 1) / P.slices : 0;
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < P.stages; i++) {
+            bar_init(&full[i], 1);
+            bar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            bar_init(&tfull[i], 1);
+            bar_init(&tempty[i], 8);
+        }
+        bar_init(&afull, 1);
+        bar_init(&done, 1);
+        stop_word = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 17) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    const uint32_t C = P.chunks, R = P.stages;
+
+    if (warp == 16) {
+        if (lane == 0) {
+            const uint8_t *ga = reinterpret_cast<const uint8_t *>(P.a) + (size_t)blockIdx.x * MB * C * kABytes;
+            bar_expect(&afull, MB * C * kABytes);
+            for (uint32_t i = 0; i < MB * C; i++) bulk_load(sa + (size_t)i * kABytes, ga + (size_t)i * kABytes, kABytes, &afull);
+            uint32_t it = 0;
+            bool ok = true;
+            for (uint32_t i = 0; ok && i < n_items; i++) {
+                const uint8_t *gb =
+                    reinterpret_cast<const uint8_t *>(P.b) + (size_t)((slice + i * P.slices) * P.stride) * C * kBBytes;
+                for (uint32_t c = 0; c < C; c++, it++) {
+                    const uint32_t st = it % R;
+                    ok = bar_wait(&empty[st], ((it / R) & 1) ^ 1, stop);
+                    if (!ok) break;
+                    bar_expect(&full[st], kBBytes);
+                    bulk_load(sb + (size_t)st * kBBytes, gb + (size_t)c * kBBytes, kBBytes, &full[st]);
+                }
+            }
+            // what is in flight ends before the block does: the last stages'
+            // releases by the MMAs, or, when a wait gave up, the copies
+            uint32_t none = 0;
+            bar_wait(&afull, 0, &none);
+            for (uint32_t b = it > R ? it - R : 0; b < it; b++) {
+                none = 0;
+                if (ok) ok = bar_wait(&empty[b % R], (b / R) & 1, stop);
+                else bar_wait(&full[b % R], (b / R) & 1, &none);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 17) {
+        // f32 accumulators, bf16 operands, both K-major, N = 256, M = 128
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | ((kBlkM >> 4) << 24);
+        const uint64_t da0 = mma_desc(smem_addr(sa)), db0 = mma_desc(smem_addr(sb));
+        const uint32_t last = P.steps - 4 * (C - 1);  // steps of the last chunk
+        // the lanes leave the loop together: a wait given up by one ends it for all
+        bool ok = __all_sync(kFull, bar_wait(&afull, 0, stop));
+        uint32_t st0 = 0, ph0 = 0;  // ring place of the tile's first chunk
+        for (uint32_t i = 0; ok && i < n_items; i++) {
+            uint32_t st = st0, ph = ph0;
+#pragma unroll
+            for (uint32_t m = 0; m < (uint32_t)MB; m++) {
+                const uint32_t buf = MB == 2 ? m : i & 1, use = MB == 2 ? i : i >> 1;
+                ok = __all_sync(kFull, ok && bar_wait(&tempty[buf], (use & 1) ^ 1, stop));
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                st = st0;
+                ph = ph0;
+                const uint32_t acc = tmem + buf * kTileN;
+                uint64_t da = da0 + (uint64_t)(m * C) * (kABytes >> 4);
+                for (uint32_t c = 0; c < C; c++) {
+                    ok = __all_sync(kFull, ok && bar_wait(&full[st], ph, stop));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t db = db0 + (uint64_t)st * (kBBytes >> 4);
+                    const uint32_t ks = c + 1 < C ? 4u : last;
+                    mma_bf16(acc, da, db, idesc, c > 0);
+                    if (ks > 1) mma_bf16(acc, da + 2, db + 2, idesc, true);
+                    if (ks > 2) mma_bf16(acc, da + 4, db + 4, idesc, true);
+                    if (ks > 3) mma_bf16(acc, da + 6, db + 6, idesc, true);
+                    if (m + 1 == (uint32_t)MB) mma_commit(&empty[st]);
+                    da += kABytes >> 4;
+                    if (++st == R) {
+                        st = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok) mma_commit(&tfull[buf]);
+            }
+            st0 = st;
+            ph0 = ph;
+        }
+        if (!ok) {  // what was issued ends before TMEM is given back
+            mma_commit(&done);
+            uint32_t none = 0;
+            bar_wait(&done, 0, &none);
+        }
+    } else {
+        // columns 128 half .. of accumulator b, rows 32 quarter ..
+        const uint32_t b = warp >> 3, half = (warp >> 2) & 1, quarter = warp & 3;
+        const uint32_t uses = MB == 2 ? n_items : (n_items + 1 - b) / 2;
+        const uint32_t q = blockIdx.x * MB * kBlkM + (MB == 2 ? b * kBlkM : 0) + quarter * 32 + lane;
+        const uint32_t t0 = tmem + ((quarter * 32) << 16) + b * kTileN + half * kHalf;
+        bool ok = true;
+        if constexpr (PASS == 1) {
+            const uint32_t part = MB == 2 ? slice : slice * 2 + b;
+            float g[32];
+#pragma unroll
+            for (int j = 0; j < 32; j++) g[j] = -3e38f;
+            for (uint32_t u = 0; ok && u < uses; u++) {
+                ok = __all_sync(kFull, bar_wait(&tfull[b], u & 1, stop));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                float v[2][32];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    tmem_ld32(t0 + 64 * h, v[0]);
+                    tmem_ld32(t0 + 64 * h + 32, v[1]);
+                    tmem_wait(v[0]);
+                    tmem_wait(v[1]);
+                    if (h == 1) {  // the accumulator is read: the next tile's MMAs may write it
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(&tempty[b]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j++) g[j] = max3(g[j], v[0][j], v[1][j]);
+                }
+            }
+            if (q < P.nq) {
+                float4 *o = reinterpret_cast<float4 *>(P.gmax + ((size_t)part * P.nq + q) * kGroups + half * 32);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    o[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+            }
+        } else {
+            const uint32_t part = (MB == 2 ? slice : slice * 2 + b) * 2 + half;
+            const float least = q < P.nq ? P.least[q] : __int_as_float(0x7f800000);
+            uint32_t *list = P.list + ((size_t)part * P.nq + (q < P.nq ? q : 0)) * P.cap;
+            uint32_t count = 0;
+            for (uint32_t u = 0; ok && u < uses; u++) {
+                ok = __all_sync(kFull, bar_wait(&tfull[b], u & 1, stop));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t item = MB == 2 ? u : 2 * u + b;
+                const uint32_t p0 = (slice + item * P.slices) * P.stride * kTileN + half * kHalf;
+                constexpr int kS = (int)kHalf / 32;
+                uint32_t hit[kS];
+                float v[2][32];
+                tmem_ld32(t0, v[0]);
+                tmem_ld32(t0 + 32, v[1]);
+#pragma unroll
+                for (int h = 0; h < kS; h++) {
+                    float(&w)[32] = v[h & 1];
+                    if (h == 0 || h == 2) {
+                        tmem_wait(v[0]);
+                        tmem_wait(v[1]);
+                    }
+                    if (h == 2) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(&tempty[b]);
+                    }
+                    float m[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        m[e] = max3(w[8 * e], w[8 * e + 1], w[8 * e + 2]);
+                        m[e] = max3(m[e], w[8 * e + 3], w[8 * e + 4]);
+                        m[e] = max3(m[e], w[8 * e + 5], w[8 * e + 6]);
+                        m[e] = fmaxf(m[e], w[8 * e + 7]);
+                    }
+                    hit[h] = 0;
+                    if (fmaxf(max3(m[0], m[1], m[2]), m[3]) >= least) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            if (m[e] >= least) {
+#pragma unroll
+                                for (int j = 0; j < 8; j++) hit[h] |= w[8 * e + j] >= least ? 1u << (8 * e + j) : 0u;
+                            }
+                    }
+                    if (h < 2) tmem_ld32(t0 + 64 + 32 * h, w);
+                }
+#pragma unroll
+                for (int h = 0; h < kS; h++)
+                    while (hit[h]) {
+                        if (count < P.cap) list[count] = p0 + 32 * h + (uint32_t)__ffs(hit[h]) - 1u;
+                        count++;
+                        hit[h] &= hit[h] - 1u;
+                    }
+            }
+            if (q < P.nq) P.count[(size_t)part * P.nq + q] = count;
+        }
+        if (!ok && lane == 0) *P.bad = 1u;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x == 0 && stop_word) *P.bad = 1u;
+    if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// The least score a true neighbour of each query can have; a warp per query.
+// v, the (k + 1)-th largest group maximum, stands for k + 1 different points,
+// at least k of them not the query itself.
+// Euclidean: such a point has distance D <= u^2 - 2 (v - E), where E =
+// kappa (u^2 + w^2) + 1e-30 and w bounds its norm (w <= u + sqrt(D), solved
+// with the bound's own share of D); a true neighbour's distance is then at
+// most D (1 + 4 gamma), gamma = (dim + 8) 2^-24 covering the chain's rounding
+// on both sides, its norm at most u + sqrt of that, its score at least (u^2 -
+// D (1 + 4 gamma)) / 2 less the bound. Cosine: scores are the dot products of
+// unit rows, E = 2.1 kappa, the chain's rounding dim 2^-24 on both sides and
+// that of 1 - dot.
+__global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t parts, uint32_t nq, uint32_t k,
+                                   const float *__restrict__ norm, const uint32_t *__restrict__ qidx, uint32_t q0,
+                                   uint32_t dim, bool euc, double kappa, float *__restrict__ least)
+{
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (q >= nq) return;  // warp-uniform
+    float v0 = -3e38f, v1 = -3e38f;
+    for (uint32_t p = 0; p < parts; p++) {
+        const float2 f = __ldcs(reinterpret_cast<const float2 *>(gmax + ((size_t)p * nq + q) * kGroups) + lane);
+        v0 = fmaxf(v0, f.x);
+        v1 = fmaxf(v1, f.y);
+    }
+    // unsigned integers in the floats' order
+    uint32_t o0 = __float_as_uint(v0), o1 = __float_as_uint(v1);
+    o0 = (o0 & 0x80000000u) ? ~o0 : o0 | 0x80000000u;
+    o1 = (o1 & 0x80000000u) ? ~o1 : o1 | 0x80000000u;
+    uint32_t top = 0;
+    for (uint32_t r = 0; r <= k; r++) {
+        const uint32_t mine = max(o0, o1);
+        top = __reduce_max_sync(kFull, mine);
+        const unsigned who = __ballot_sync(kFull, mine == top);
+        if ((int)lane == __ffs(who) - 1) {
+            if (o0 == top) o0 = 0;
+            else o1 = 0;
+        }
+    }
+    if (lane != 0) return;
+    const double s = (double)__uint_as_float((top & 0x80000000u) ? top ^ 0x80000000u : ~top);
+    double g;
+    if (euc) {
+        const double u2 = (double)norm[qidx ? qidx[q0 + q] : q0 + q], u = sqrt(u2), tiny = 1e-30;
+        const double d0 = fmax(u2 - 2.0 * s, 0.0);
+        const double w = (u + sqrt(d0 + 2.0 * kappa * u2 + tiny)) / (1.0 - sqrt(2.0 * kappa));
+        const double d1 = (d0 + 2.0 * (kappa * (u2 + w * w) + tiny)) * (1.0 + 4.0 * (dim + 8) * 0x1p-24);
+        const double w1 = u + sqrt(d1);
+        g = 0.5 * (u2 - d1) - kappa * (u2 + w1 * w1) - 2.0 * tiny;
+    } else {
+        g = s - 2.0 * 2.1 * kappa - (2.0 * dim + 16.0) * 0x1p-24 - 0x1p-22;
+    }
+    least[q] = __double2float_rd(g);
+}
+
+__device__ __forceinline__ bool better(float d, uint32_t i, float td, uint32_t ti)
+{
+    return d < td || (d == td && i < ti);
+}
+
+// The exact second look, a warp per query: 32 candidates at a time, their
+// rows staged through shared memory 32 dims at a time (coalesced; a lane
+// reading its own candidate's row would touch 32 lines a load), the distance
+// chain of knn.cu per lane, and insertion into the warp's sorted list (lane l
+// holds entry l). A query whose lists overflowed, or any query when *bad, goes
+// to left.
+constexpr int kRefineWarps = 4;
+template <bool EUC>
+__global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__restrict__ x, uint32_t n, uint32_t dim, uint32_t k,
+                                                              const uint32_t *__restrict__ qidx, uint32_t q0,
+                                                              uint32_t nq, const uint32_t *__restrict__ list,
+                                                              const uint32_t *__restrict__ count, uint32_t parts,
+                                                              uint32_t cap, const uint32_t *__restrict__ bad,
+                                                              uint32_t *__restrict__ out_idx,
+                                                              float *__restrict__ out_dist,
+                                                              uint32_t *__restrict__ left, uint32_t *__restrict__ n_left)
+{
+    __shared__ float sh[kRefineWarps][32][33];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t q = blockIdx.x * kRefineWarps + warp;
+    if (q >= nq) return;  // warp-uniform
+    float(&S)[32][33] = sh[warp];
+    const uint32_t self = qidx ? qidx[q0 + q] : q0 + q;
+    const float *xq = x + (size_t)self * dim;
+    bool over = *bad != 0;
+    float ld = __int_as_float(0x7f800000);
+    uint32_t li = ~0u;
+    for (uint32_t p = 0; !over && p < parts; p++) {
+        const uint32_t c = count[(size_t)p * nq + q];
+        if (c > cap) {
+            over = true;
+            break;
+        }
+        const uint32_t *L = list + ((size_t)p * nq + q) * cap;
+        for (uint32_t b = 0; b < c; b += 32) {
+            bool live = b + lane < c;
+            uint32_t mine = live ? L[b + lane] : self;
+            if (mine >= n) {  // the last tile's padding, listed only under a threshold that excludes nothing
+                live = false;
+                mine = self;
+            }
+            const uint32_t rows = min(32u, c - b);
+            float acc = 0.0f;
+            for (uint32_t d0 = 0; d0 < dim; d0 += 32) {
+                const uint32_t w = min(32u, dim - d0);
+                __syncwarp();
+                if (w > 16) {
+#pragma unroll 8
+                    for (uint32_t r = 0; r < rows; r++) {
+                        const uint32_t id = __shfl_sync(kFull, mine, r);
+                        if (lane < w) S[r][lane] = __ldg(x + (size_t)id * dim + d0 + lane);
+                    }
+                } else {  // two rows a step
+                    for (uint32_t r = 0; r < rows; r += 2) {
+                        const uint32_t id = __shfl_sync(kFull, mine, (r + (lane >> 4)) & 31u);
+                        const uint32_t e = lane & 15;
+                        if (e < w) S[r + (lane >> 4)][e] = __ldg(x + (size_t)id * dim + d0 + e);
+                    }
+                }
+                __syncwarp();
+                for (uint32_t d = 0; d < w; d++) {
+                    const float a = __ldg(xq + d0 + d), v = S[lane][d];
+                    if (EUC) {
+                        const float df = a - v;
+                        acc = __fmaf_rn(df, df, acc);
+                    } else {
+                        acc = __fmaf_rn(a, v, acc);
+                    }
+                }
+            }
+            const float dist = EUC ? acc : 1.0f - acc;
+            float td = __shfl_sync(kFull, ld, k - 1);
+            uint32_t ti = __shfl_sync(kFull, li, k - 1);
+            unsigned pend = __ballot_sync(kFull, live && mine != self && better(dist, mine, td, ti));
+            while (pend) {
+                const int src = __ffs(pend) - 1;
+                pend &= pend - 1;
+                const float cd = __shfl_sync(kFull, dist, src);
+                const uint32_t ci = __shfl_sync(kFull, mine, src);
+                const uint32_t pos = __popc(__ballot_sync(kFull, better(ld, li, cd, ci)));
+                const float ud = __shfl_up_sync(kFull, ld, 1);
+                const uint32_t ui = __shfl_up_sync(kFull, li, 1);
+                if (lane < k) {
+                    if (lane > pos) {
+                        ld = ud;
+                        li = ui;
+                    } else if (lane == pos) {
+                        ld = cd;
+                        li = ci;
+                    }
+                }
+            }
+        }
+    }
+    if (!over && __shfl_sync(kFull, li, k - 1) == ~0u) over = true;  // fewer than k: never with a true bound
+    if (over) {
+        if (lane == 0) left[atomicAdd(n_left, 1u)] = q0 + q;
+    } else if (lane < k) {
+        out_idx[(size_t)(q0 + q) * k + lane] = li;
+        out_dist[(size_t)(q0 + q) * k + lane] = ld;
+    }
+}
+
+template <int MB, int PASS>
+void launch_filter(const FilterArgs &P, uint32_t blocks, size_t smem, cudaStream_t s)
+{
+    check_cuda(cudaFuncSetAttribute(k_filter<MB, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+               "filter shared memory");
+    k_filter<MB, PASS><<<dim3(blocks, P.slices), kFilterThreads, smem, s>>>(P);
+    check_launch("k_filter");
+}
+
+}  // namespace
+
+// The filter's fixed cost (packing, eight launches) is some tens of
+// microseconds, so it takes searches of at least kFilterPairs pairs; below
+// kFilterPoints points the sample is too small for its groups, and beyond 191
+// dims the operands no longer fit beside the ring.
+bool knn_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k)
+{
+    constexpr uint32_t kFilterPoints = 2048;
+    constexpr uint64_t kFilterPairs = 4u << 20;
+    return n >= kFilterPoints && (uint64_t)n * nq >= kFilterPairs && pack_of(dim).chunks <= kMaxChunks &&
+           n < (1u << 30) && k + 1 < kGroups;
+}
+
+bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaStream_t s)
+{
+    const Pack pk = pack_of(A.dim);
+    const uint32_t C = pk.chunks, MB = C <= 3 ? 2 : 1;
+    const uint32_t n_tiles = ceil_div(A.n, kTileN), sms = (uint32_t)device_sm_count();
+    const uint32_t stages = std::min<uint32_t>(5, (kSmemMax - 2048 - MB * C * kABytes) / kBBytes);
+    const size_t smem = (size_t)MB * C * kABytes + (size_t)stages * kBBytes + 1024;
+    // every stride-th tile: the sample's (k + 1)-th group maximum is about its
+    // r-th best point, r = -G ln(1 - (k + 1) / G), so about r * stride
+    // points of all reach it
+    const double r = -(double)kGroups * std::log(1.0 - (double)(A.k + 1) / kGroups);
+    const uint32_t stride = std::max(1u, std::min((uint32_t)(kHitTarget / r), n_tiles / 4));
+    // queries in batches of at most two waves of blocks: bounds the scratch
+    const uint32_t rows = MB * kBlkM, batch = std::min<uint32_t>(ceil_div(A.nq, rows), 2 * MB == 4 ? 2 * sms : 4 * sms) * rows;
+    // slices of the points: fewest rounds of blocks over the SMs, a block
+    // costing about six tiles besides its own
+    auto slices_of = [&](uint32_t blocks, uint32_t tiles) {
+        uint32_t best = 1;
+        uint64_t cost = ~0ull;
+        for (uint32_t S = 1; S <= 16 && S <= tiles; S++) {
+            const uint64_t c = (uint64_t)ceil_div((uint64_t)blocks * S, sms) * (ceil_div(tiles, S) + 6);
+            if (c < cost) {
+                cost = c;
+                best = S;
+            }
+        }
+        return best;
+    };
+    const uint32_t sampled = ceil_div(n_tiles, stride);
+    uint32_t most1 = 1, most2 = 1;
+    for (uint32_t q0 = 0; q0 < A.nq; q0 += batch) {
+        const uint32_t blocks = ceil_div(std::min(batch, A.nq - q0), rows);
+        most1 = std::max(most1, slices_of(blocks, sampled) * blocks);
+        most2 = std::max(most2, slices_of(blocks, n_tiles) * blocks);
+    }
+    const uint32_t per = MB == 2 ? 1 : 2;  // accumulators of a slice
+    DevBuf<float> mu, norm, gmax, least;
+    DevBuf<uint4> pa, pb;
+    DevBuf<uint32_t> list, count, bad;
+    try {
+        mu.alloc(A.dim, s);
+        norm.alloc(A.n, s);
+        pb.alloc((size_t)n_tiles * C * (kBBytes / 16), s);
+        pa.alloc((size_t)(batch / kBlkM) * C * (kABytes / 16), s);
+        gmax.alloc((size_t)most1 * per * rows * kGroups, s);
+        least.alloc(batch, s);
+        // a part's list (a slice's, of one half of the columns) holds its
+        // share of kListCap and 64 more
+        list.alloc((size_t)most2 * per * 2 * rows * 64 + (size_t)batch * kListCap, s);
+        count.alloc((size_t)most2 * per * 2 * rows, s);
+        bad.alloc(1, s);
+    } catch (const Error &e) {
+        if (e.status != UMAPCU_CUDA_ALLOC) throw;
+        return false;
+    }
+    check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
+    const float *centre = nullptr;
+    if (A.euc) {
+        k_filter_centre<<<ceil_div(A.dim, 8), 1024, 0, s>>>(A.x, A.n, A.dim, mu.p);
+        centre = mu.p;
+    }
+    k_filter_norms<<<ceil_div((uint64_t)A.n * 32, 256), 256, 0, s>>>(A.x, A.n, A.dim, centre, norm.p, bad.p);
+    k_filter_pack<false><<<ceil_div((uint64_t)n_tiles * kTileN * C * 8, 256), 256, 0, s>>>(
+        A.x, A.n, A.dim, centre, norm.p, nullptr, 0, A.n, n_tiles * kTileN, pk.terms, C, A.euc, pb.p);
+    check_launch("filter packing");
+    for (uint32_t q0 = 0; q0 < A.nq; q0 += batch) {
+        const uint32_t nq = std::min(batch, A.nq - q0), blocks = ceil_div(nq, rows);
+        k_filter_pack<true><<<ceil_div((uint64_t)blocks * rows * C * 8, 256), 256, 0, s>>>(
+            A.x, A.n, A.dim, centre, norm.p, A.qidx, q0, nq, blocks * rows, pk.terms, C, A.euc, pa.p);
+        FilterArgs P{};
+        P.a = pa.p;
+        P.b = pb.p;
+        P.nq = nq;
+        P.n_tiles = n_tiles;
+        P.chunks = C;
+        P.steps = pk.steps;
+        P.stages = stages;
+        P.bad = bad.p;
+        P.stride = stride;
+        P.slices = slices_of(blocks, sampled);
+        P.gmax = gmax.p;
+        if (MB == 2) launch_filter<2, 1>(P, blocks, smem, s);
+        else launch_filter<1, 1>(P, blocks, smem, s);
+        k_filter_threshold<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(
+            gmax.p, P.slices * per, nq, A.k, norm.p, A.qidx, q0, A.dim, A.euc, filter_kappa(pk.terms), least.p);
+        check_launch("k_filter_threshold");
+        P.stride = 1;
+        P.slices = slices_of(blocks, n_tiles);
+        P.least = least.p;
+        P.list = list.p;
+        P.count = count.p;
+        const uint32_t parts = P.slices * per * 2;
+        P.cap = kListCap / parts + 64;
+        if (MB == 2) launch_filter<2, 2>(P, blocks, smem, s);
+        else launch_filter<1, 2>(P, blocks, smem, s);
+        const unsigned rg = ceil_div(nq, kRefineWarps);
+        if (A.euc)
+            k_refine<true><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, list.p, count.p, parts,
+                                                            P.cap, bad.p, A.out_idx, A.out_dist, left, n_left);
+        else
+            k_refine<false><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, list.p, count.p, parts,
+                                                             P.cap, bad.p, A.out_idx, A.out_dist, left, n_left);
+        check_launch("k_refine");
+    }
+    return true;
+}
+
+}  // namespace umapcu
