@@ -48,6 +48,10 @@ struct umapcu_state {
     ScheduleLists lists;
     ScheduleBits bits;  // the bitmask form, used when there are no lists
     DevBuf<uint32_t> err;  // checked builds: a kernel's report of a bad index
+    // layout_resident.cu: status and the epochs' counters, their scalars, the rows
+    DevBuf<uint32_t> meet;
+    DevBuf<float4> scal;
+    DevBuf<uint4> ring;
     bool lists_ok = false, bits_ok = false, sched_continuous = true, sched_lazy = false;
     uint32_t sched_epoch = 0;
     float lists_build_ms = 0.0f;
@@ -131,32 +135,10 @@ umapcu_status take_error(umapcu_state *st)
 #endif
 }
 
-void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint32_t *d_inj, float *d_grad,
-               uint32_t *d_act, bool skip_dens = false)
+// An epoch's arguments but for its schedule and debug outputs.
+EpochArgs epoch_args(umapcu_state *st, uint32_t epoch, uint32_t optimiser)
 {
-    const bool dens_on = st->dens && dens_active(st->lambda, st->frac, epoch, st->p.n_epochs);
-    if (dens_on && !skip_dens) dens_update(st);
-    const bool in_order = st->sched_continuous && epoch == st->sched_epoch;
-    const bool use_lists = st->lists_ok && in_order && epoch < st->lists.n_epochs;
-    const bool use_bits = !use_lists && st->bits_ok && in_order && epoch < st->bits.n_epochs;
-    if (!use_lists && !use_bits) sync_cursors(st);  // the scan reads and advances the cursors
-    if (!in_order) st->sched_continuous = false;
     EpochArgs A{};
-    if (use_lists) {
-        A.rec = st->lists.rec.p;
-        A.seg_ptr = st->lists.ptr.p + (size_t)epoch * st->lists.n_units;
-        A.seg_unit = st->lists.unit_base.p;
-        st->sched_lazy = true;
-    } else if (use_bits) {
-        A.bits = st->bits.bits + (size_t)epoch * st->bits.words;
-        st->sched_lazy = true;
-        if (st->bits.rest && epoch >= st->bits.first && st->bits.waited != st->stream.s) {
-            // the later epochs' words (build_schedule_bits): once per stream
-            check_cuda(cudaStreamWaitEvent(st->stream.s, st->bits.rest, 0), "cudaStreamWaitEvent");
-            st->bits.waited = st->stream.s;
-        }
-    }
-    if (in_order) st->sched_epoch = epoch + 1;
     A.n = st->n;
     A.offsets = st->csr.offsets.p;
     A.other = st->csr.other.p;
@@ -168,9 +150,6 @@ void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint3
     A.v = st->v.p;
     A.dens_node = st->dens_node.p;
     A.dens_stats = st->stats.p;
-    A.injected = d_inj;
-    A.dbg_grad = d_grad;
-    A.dbg_active = d_act;
     A.epoch = epoch;
     A.epoch_f = (float)epoch;
     epoch_scalars(st->p, epoch, &A.fused, &A.epsc, &A.lr_sgd);
@@ -190,8 +169,88 @@ void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint3
     A.precise_pow = st->precise_pow;
     A.n_entries = 2 * st->csr.n_edges;
     A.err = st->err.p;
+    return A;
+}
+
+// The words build_schedule_bits left to its side stream: waited for once per
+// stream.
+void wait_bits(umapcu_state *st)
+{
+    if (!st->bits.rest || st->bits.waited == st->stream.s) return;
+    check_cuda(cudaStreamWaitEvent(st->stream.s, st->bits.rest, 0), "cudaStreamWaitEvent");
+    st->bits.waited = st->stream.s;
+}
+
+void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint32_t *d_inj, float *d_grad,
+               uint32_t *d_act, bool skip_dens = false)
+{
+    const bool dens_on = st->dens && dens_active(st->lambda, st->frac, epoch, st->p.n_epochs);
+    if (dens_on && !skip_dens) dens_update(st);
+    const bool in_order = st->sched_continuous && epoch == st->sched_epoch;
+    const bool use_lists = st->lists_ok && in_order && epoch < st->lists.n_epochs;
+    const bool use_bits = !use_lists && st->bits_ok && in_order && epoch < st->bits.n_epochs;
+    if (!use_lists && !use_bits) sync_cursors(st);  // the scan reads and advances the cursors
+    if (!in_order) st->sched_continuous = false;
+    EpochArgs A = epoch_args(st, epoch, optimiser);
+    if (use_lists) {
+        A.rec = st->lists.rec.p;
+        A.seg_ptr = st->lists.ptr.p + (size_t)epoch * st->lists.n_units;
+        A.seg_unit = st->lists.unit_base.p;
+        st->sched_lazy = true;
+    } else if (use_bits) {
+        A.bits = st->bits.bits + (size_t)epoch * st->bits.words;
+        st->sched_lazy = true;
+        if (epoch >= st->bits.first) wait_bits(st);
+    }
+    if (in_order) st->sched_epoch = epoch + 1;
+    A.injected = d_inj;
+    A.dbg_grad = d_grad;
+    A.dbg_active = d_act;
     launch_epoch(A, st->n_dim, dens_on, st->stream.s);
     st->cur ^= 1;
+}
+
+// Epochs [first, last) of a run on bitmasks; spans of epochs without the
+// density term in one launch where layout_resident.cu takes them (a span of a
+// few epochs gains nothing over launches). true: a resident launch was made,
+// and st->meet's status is to be looked at once it has run.
+bool run_epochs(umapcu_state *st, uint32_t first, uint32_t last, uint32_t optimiser, bool resident)
+{
+    constexpr uint32_t kSpan = 4;
+    bool used = false;
+    resident = resident && st->bits_ok && !st->lists_ok && last <= st->bits.n_epochs && !st->precise_pow &&
+               st->sampler == UMAPCU_NEG_REF_HASH && st->p.neg_sample_rate == 5 && resident_takes(st->n, st->n_dim);
+    for (uint32_t e = first; e < last;) {
+        uint32_t end = e;
+        while (end < last && !(st->dens && dens_active(st->lambda, st->frac, end, st->p.n_epochs))) end++;
+        if (resident && end - e >= kSpan && st->sched_continuous && e == st->sched_epoch) {
+            std::vector<float4> sc(end - e);
+            for (uint32_t i = 0; i < sc.size(); i++) epoch_scalars(st->p, e + i, &sc[i].x, &sc[i].y, &sc[i].z);
+            cudaStream_t s = st->stream.s;
+            if (!st->meet.p) {
+                st->meet.alloc((size_t)st->p.n_epochs + 1, s);
+                check_cuda(cudaMemsetAsync(st->meet.p, 0, sizeof(uint32_t), s), "memset status");
+            }
+            st->scal.alloc(sc.size(), s);
+            h2d(st->scal.p, sc.data(), sc.size(), s);
+            if (!st->ring.p) st->ring.alloc(resident_ring_bytes(st->n) / sizeof(uint4), s);
+            wait_bits(st);
+            EpochArgs A = epoch_args(st, e, optimiser);
+            A.bits = st->bits.bits;
+            if (launch_layout_resident(A, st->n_dim, st->scal.p, e, end - e, st->bits.words, st->ring.p,
+                                       st->meet.p + 1, st->meet.p, s)) {
+                used = true;
+                st->cur ^= (end - e) & 1;
+                st->sched_epoch = end;
+                st->sched_lazy = true;
+                e = end;
+                continue;
+            }
+            resident = false;
+        }
+        run_epoch(st, e++, optimiser, nullptr, nullptr, nullptr);
+    }
+    return used;
 }
 
 // Optional phase timing of the host-buffer entry points (UMAPCU_TIMING=1):
@@ -785,20 +844,40 @@ umapcu_status umapcu_optimise_embedding(float *embd, uint32_t n, uint32_t n_dim,
         const uint64_t nt = (uint64_t)n * n_dim;
         PhaseTimer T;
         NvtxRange r("umapcu epochs");
-        for (uint32_t e = 0; e < params->n_epochs; e++) {
-            const bool log_now = verbose && ((e + 1) % 100 == 0 || e + 1 == params->n_epochs);
-            if (!log_now) {
-                run_epoch(st.get(), e, optimiser, nullptr, nullptr, nullptr);
-                continue;
+        auto run_all = [&](bool resident) {
+            bool used = false;
+            for (uint32_t e = 0; e < params->n_epochs;) {
+                uint32_t log = params->n_epochs;  // the next epoch whose gradient norm is printed
+                if (verbose) log = std::min(params->n_epochs - 1, e / 100 * 100 + 99);
+                used = run_epochs(st.get(), e, log, optimiser, resident) || used;
+                e = log;
+                if (e == params->n_epochs) break;
+                DevBuf<float> g(nt, st->stream.s);
+                run_epoch(st.get(), e, optimiser, nullptr, g.p, nullptr);
+                std::vector<float> hg(nt);
+                d2h(hg.data(), g.p, nt, st->stream.s);
+                sync(st->stream.s);
+                double ss = 0.0;
+                for (float x : hg) ss += (double)x * x;
+                printf(" Epoch %u / %u: grad norm %.2f\n", e + 1, params->n_epochs, sqrt(ss));
+                e++;
             }
-            DevBuf<float> g(nt, st->stream.s);
-            run_epoch(st.get(), e, optimiser, nullptr, g.p, nullptr);
-            std::vector<float> hg(nt);
-            d2h(hg.data(), g.p, nt, st->stream.s);
+            return used;
+        };
+        if (run_all(true)) {
+            uint32_t status = 0;
+            d2h(&status, st->meet.p, 1, st->stream.s);
             sync(st->stream.s);
-            double ss = 0.0;
-            for (float x : hg) ss += (double)x * x;
-            printf(" Epoch %u / %u: grad norm %.2f\n", e + 1, params->n_epochs, sqrt(ss));
+            if (status) {  // a segment too long, or a wait that gave up: once more, a launch per epoch
+                cudaStream_t s = st->stream.s;
+                st->cur = 0;
+                h2d(st->y[0].p, embd, nt, s);
+                check_cuda(cudaMemsetAsync(st->m.p, 0, nt * sizeof(float), s), "memset m");
+                check_cuda(cudaMemsetAsync(st->v.p, 0, nt * sizeof(float), s), "memset v");
+                st->sched_epoch = 0;
+                st->sched_continuous = true;
+                run_all(false);
+            }
         }
         T.mark("epochs", st->stream.s);
         d2h(embd, st->y[st->cur].p, nt, st->stream.s);

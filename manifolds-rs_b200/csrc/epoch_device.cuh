@@ -246,6 +246,13 @@ __device__ __forceinline__ uint32_t local_node(const uint32_t *beg, uint32_t p)
     return j;
 }
 
+// An entry's gathered rows: the other endpoint's and its negatives'.
+template <int D, int NR>
+struct BatchRows {
+    uint32_t kk[NR > 0 ? NR : 1];
+    float yo[D], yk[NR > 0 ? NR : 1][D];
+};
+
 // One batch of up to 32 active entries, lane t = entry t (`live` lanes
 // only): CSR position p, other endpoint o, the entry's node as an index j
 // into the segment, and its offset el within the node's row. The other
@@ -256,12 +263,15 @@ __device__ __forceinline__ uint32_t local_node(const uint32_t *beg, uint32_t p)
 // removes the per-negative and per-term uniform branches of the general path.
 // The batch's per-node sums go to part[j] for the nodes in the returned
 // mask; unless SPLIT, the node's lane then adds them to g (and sets act).
-template <int D, bool DENS, int NR, bool COH, int KU, bool FAST, bool SPLIT = false, class Smem = WarpSmem<D, KU>>
+// PRE: the entry's negatives and all its rows come in pre (FAST, NR > 0 only).
+template <int D, bool DENS, int NR, bool COH, int KU, bool FAST, bool SPLIT = false, bool PRE = false,
+          class Smem = WarpSmem<D, KU>>
 __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, bool live, uint32_t p,
                                                   uint32_t o, uint32_t j, uint32_t edge_local, uint32_t node0,
                                                   int lane, float (&g)[D], bool &act, const float *dstat,
-                                                  float (*part)[D])
+                                                  float (*part)[D], const BatchRows<D, NR> *pre = nullptr)
 {
+    static_assert(!PRE || (FAST && NR > 0 && !DENS), "rows in advance: the fast path");
     if (live && !checked_ok(o < A.n && p < A.n_entries, A.err)) live = false;
     if (!live) j = 32;  // dead lanes: a node of their own, contributing zero
     float c[D];
@@ -285,6 +295,12 @@ __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, b
             for (int t = 0; t < kNegChunk; t++) {
                 const uint32_t neg = k0 + t;
                 uint32_t kn = self;
+                if constexpr (PRE) {
+                    kk[t] = pre->kk[t];
+#pragma unroll
+                    for (int d = 0; d < D; d++) yk[t][d] = pre->yk[t][d];
+                    continue;
+                }
                 if (neg < neg_rate) {
                     if (!FAST && A.injected) {
                         kn = A.injected[(uint64_t)p * neg_rate + neg];
@@ -302,9 +318,14 @@ __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, b
                 if (neg < neg_rate) load_row_keep<D, COH>(A.y_cur, kn, yk[t], pol);
             }
         };
-        load_row_keep<D, COH>(A.y_cur, o, yo, pol);
+        if constexpr (PRE) {
+#pragma unroll
+            for (int d = 0; d < D; d++) yo[d] = pre->yo[d];
+        } else {
+            load_row_keep<D, COH>(A.y_cur, o, yo, pol);
+        }
         // (wider rows: registers for all gathers at once would spill)
-        if constexpr (D <= 2) issue(0);
+        if constexpr (D <= 2 || PRE) issue(0);
         float4 dno;
         float mu_e = 1.0f;
         if constexpr (DENS) {
@@ -348,7 +369,30 @@ __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, b
         }
         // negatives (umap_optimiser_gpu.rs:817-849)
         for (uint32_t k0 = 0; k0 < neg_rate; k0 += kNegChunk) {
-            if (k0 || D > 2) issue(k0);
+            if (k0 || (D > 2 && !PRE)) issue(k0);
+            if constexpr (PRE) {
+                // a lone warp's latency counts here: the negatives' chains run
+                // side by side, without a branch for each
+                float gc[kNegChunk], diff[kNegChunk][D];
+#pragma unroll
+                for (int t = 0; t < kNegChunk; t++) {
+                    float dsk = 0.0f;
+#pragma unroll
+                    for (int d = 0; d < D; d++) {
+                        diff[t][d] = ys[d] - yk[t][d];
+                        dsk += diff[t][d] * diff[t][d];
+                    }
+                    const float dist_sq_safe = dsk + 0.001f;
+                    const float dist_sq_b = pow_pos(dist_sq_safe, A.b, false);
+                    const float denom = dist_sq_safe * (1.0f + A.a * dist_sq_b);
+                    gc[t] = clip4(div_k(A.two_gamma_b, denom, false));
+                }
+#pragma unroll
+                for (int t = 0; t < kNegChunk; t++)
+#pragma unroll
+                    for (int d = 0; d < D; d++) c[d] = kk[t] != self ? c[d] + gc[t] * diff[t][d] : c[d];
+                continue;
+            }
 #pragma unroll
             for (int t = 0; t < kNegChunk; t++) {
                 if (k0 + t < neg_rate && kk[t] != self) {
