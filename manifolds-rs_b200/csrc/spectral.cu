@@ -34,17 +34,33 @@ namespace {
 
 constexpr int kBlk = 256;
 
-// y = M x, one warp per row, f64
+// y = M x, f64, eight lanes per row (a row of a kNN graph has some 25 entries:
+// with a warp per row most of the latency was spent on a quarter of the lanes;
+// 24 -> 16 us at 100k rows, 2.3M entries, caches cold), four entries of a lane in flight.
+constexpr uint32_t kRowLanes = 8;
 __global__ void k_spmv(uint32_t n, const uint64_t *__restrict__ ptr, const uint32_t *__restrict__ col,
                        const double *__restrict__ val, const double *__restrict__ x, double *__restrict__ y)
 {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kRowLanes, lane = t % kRowLanes;
     double acc = 0.0;
-    for (uint64_t p = ptr[row] + lane; p < ptr[row + 1]; p += 32) acc += val[p] * x[col[p]];
+    if (row < n) {
+        const uint64_t end = ptr[row + 1];
+        for (uint64_t p = ptr[row] + lane; p < end; p += 4 * kRowLanes) {
+            double v[4], u[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o);
-    if (lane == 0) y[row] = acc;
+            for (int i = 0; i < 4; i++) {
+                const uint64_t q = p + (uint64_t)i * kRowLanes;
+                v[i] = q < end ? val[q] : 0.0;
+                u[i] = q < end ? x[col[q]] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (p + (uint64_t)i * kRowLanes < end) acc += v[i] * u[i];
+        }
+    }
+#pragma unroll
+    for (int o = kRowLanes / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o, kRowLanes);
+    if (row < n && lane == 0) y[row] = acc;
 }
 
 // Partial dot products for long vectors: block (b, j) sums a grid-strided
@@ -100,12 +116,14 @@ __global__ void k_scale_by(const double *__restrict__ x, uint32_t n, const doubl
     dst[i] = nr > 0.0 ? x[i] / nr : x[i];
 }
 
-// c [0..j] = (0, ..., beta_{j-1}, alpha_j) from ab (alpha_i = ab[2i],
-// beta_i^2 = ab[2i + 1])
+// c = (beta_{j-1}, alpha_j), or (alpha_0) for j = 0, from ab (alpha_i =
+// ab[2i], beta_i^2 = ab[2i + 1])
 __global__ void k_recurrence_coef(const double *__restrict__ ab, uint32_t j, double *__restrict__ c)
 {
-    for (uint32_t i = threadIdx.x; i <= j; i += blockDim.x)
-        c[i] = i == j ? ab[2 * j] : (i + 1 == j ? sqrt(ab[2 * i + 1]) : 0.0);
+    if (threadIdx.x == 0) {
+        c[j ? 1 : 0] = ab[2 * j];
+        if (j) c[0] = sqrt(ab[2 * j - 1]);
+    }
 }
 
 // Start vector: uniform in [-0.5, 0.5) from a counter-based SplitMix64
@@ -205,11 +223,12 @@ void smallest_eigenpairs_dev(uint32_t n, const uint64_t *d_ptr, const uint32_t *
     check_launch("start vector");
     for (uint32_t j = 0; j < n_iter; j++) {
         double *vj = V.p + (size_t)j * n;
-        k_spmv<<<ceil_div((uint64_t)n * 32, kBlk), kBlk, 0, s>>>(n, d_ptr, d_col, d_val, vj, w.p);
+        k_spmv<<<ceil_div((uint64_t)n * kRowLanes, kBlk), kBlk, 0, s>>>(n, d_ptr, d_col, d_val, vj, w.p);
         basis_dots(vj, n, 1, w.p, part.p, ab.p + 2 * j, s);  // alpha_j
         // w -= alpha_j v_j + beta_{j-1} v_{j-1}
+        const uint32_t r0 = j ? j - 1 : 0;
         k_recurrence_coef<<<1, 32, 0, s>>>(ab.p, j, c.p);
-        k_basis_comb<<<g, kBlk, 0, s>>>(V.p, n, j + 1, c.p, w.p, true);
+        k_basis_comb<<<g, kBlk, 0, s>>>(V.p + (size_t)r0 * n, n, j + 1 - r0, c.p, w.p, true);
         // full reorthogonalisation: two classical Gram-Schmidt passes
         for (int pass = 0; pass < 2; pass++) {
             basis_dots(V.p, n, j + 1, w.p, part.p, c.p, s);
@@ -310,111 +329,278 @@ __global__ void k_neg_norm_values(uint32_t n, const uint64_t *__restrict__ ptr, 
 
 // ---- batched Lanczos: every component's recurrence advances together.
 // The normalised adjacency of the whole graph is block-diagonal (no edge
-// crosses components), so one SpMV serves all of them; the per-component
-// dot products run over each component's member list (mem[seg[s] ..
-// seg[s + 1]]) as fixed-order partial sums; sidx[g] is point g's segment
-// (~0: not solved, its vector entries stay zero).
-// Per-component dot products over the whole index space: every component
-// (segment) is cut into chunks of at most kSegChunk of its members, one block
-// per (chunk, row); a segment's chunks are consecutive work items
-// [pofs[s], pofs[s + 1]) and are summed in order, so the result does not
-// depend on scheduling.
-constexpr uint32_t kSegChunk = 4096;
+// crosses components), so one SpMV serves all of them. The solved components'
+// points are renumbered component by component (segments), members in
+// ascending order, and the matrix with them: every vector is then contiguous
+// per segment. (In the points' own order, which is unrelated to the components,
+// the dot products gathered 8 bytes from a 32-byte sector each: 14 -> 5.5 us
+// a launch at 100k points, caches cold.)
+// Per-component dot products are fixed-order partial sums: every segment is cut
+// into chunks of at most kSegChunk of its members, one block per (chunk, row);
+// a segment's chunks are consecutive work items [pofs[s], pofs[s + 1]), summed
+// in order, so the result does not depend on scheduling. sidx[g] is point g's
+// segment.
+constexpr uint32_t kSegChunk = 8 * kBlk;
 
-// part[r * n_items + t] = <V_r, w> over work item t's members
+// part[r * n_items + t] = <V_r, w> over work item t's points
 __global__ void k_seg_dots_part(const double *__restrict__ V, uint64_t n, const double *__restrict__ w,
-                                const uint32_t *__restrict__ mem, const uint32_t *__restrict__ item_beg,
-                                const uint32_t *__restrict__ item_end, uint32_t n_items, double *__restrict__ part)
+                                const uint32_t *__restrict__ item_beg, const uint32_t *__restrict__ item_end, uint32_t n_items,
+                                double *__restrict__ part)
 {
-    __shared__ double sh[kBlk];
+    __shared__ double sh[kBlk / 32];
     const uint32_t t = blockIdx.x, r = blockIdx.y;
     const double *v = V + (size_t)r * n;
+    // the thread's eight members all in flight
+    const uint32_t i0 = item_beg[t] + threadIdx.x, end = item_end[t];
+    double x[8], y[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t g = i0 + i * kBlk;
+        x[i] = g < end ? v[g] : 0.0;
+        y[i] = g < end ? w[g] : 0.0;
+    }
     double acc = 0.0;
-    for (uint32_t i = item_beg[t] + threadIdx.x; i < item_end[t]; i += kBlk) {
-        const uint32_t g = mem[i];
-        acc += v[g] * w[g];
-    }
-    sh[threadIdx.x] = acc;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) acc += x[i] * y[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
     __syncthreads();
-    for (int h = kBlk / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        double tot = 0.0;
+        for (int i = 0; i < kBlk / 32; i++) tot += sh[i];
+        part[(size_t)r * n_items + t] = tot;
     }
-    if (threadIdx.x == 0) part[(size_t)r * n_items + t] = sh[0];
 }
 
-// out[r * S + s] = sum of segment s's work items of row r, in order
+// out[r * S + s] = sum of segment s's work items of row r, a warp each, in a
+// fixed order
 __global__ void k_seg_sum_parts(const double *__restrict__ part, uint32_t n_items, const uint32_t *__restrict__ pofs,
                                 uint32_t S, uint32_t rows, double *__restrict__ out)
 {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)rows * S) return;
+    const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (t >= (uint64_t)rows * S) return;  // warp-uniform
     const uint32_t r = (uint32_t)(t / S), sg = (uint32_t)(t - (uint64_t)r * S);
     double acc = 0.0;
-    for (uint32_t q = pofs[sg]; q < pofs[sg + 1]; q++) acc += part[(size_t)r * n_items + q];
-    out[t] = acc;
+    for (uint32_t q = pofs[sg] + lane; q < pofs[sg + 1]; q += 32) acc += part[(size_t)r * n_items + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o);
+    if (lane == 0) out[t] = acc;
 }
 
-// w[g] -= sum_{r < m} c[r * S + s] V_r[g] (sub), or w[g] = that sum, for the
-// points of solved segments
+// w[g] -= sum_{r < m} c[r * S + s] V_r[g] (sub), or w[g] = that sum
 __global__ void k_seg_comb(const double *__restrict__ V, uint64_t n, uint32_t m, const double *__restrict__ c,
                            uint32_t S, const uint32_t *__restrict__ sidx, double *__restrict__ w, bool sub)
 {
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t sg = sidx[g];
-    if (sg == ~0u) return;
     double acc = 0.0;
+#pragma unroll 8
     for (uint32_t r = 0; r < m; r++) acc += c[(size_t)r * S + sg] * V[(size_t)r * n + g];
     w[g] = sub ? w[g] - acc : acc;
 }
 
-// recurrence coefficients of step j: c[r][s] = alpha_j(s) at r = j,
-// beta_{j-1}(s) at r = j - 1, else 0; ab = [step][2][S] (alpha, beta^2)
-__global__ void k_seg_recurrence(const double *__restrict__ ab, uint32_t j, uint32_t S, double *__restrict__ c)
+// recurrence of step j: w[g] -= beta_{j-1}(s) v_{j-1}[g] + alpha_j(s) v_j[g];
+// ab = [step][2][S] (alpha, beta^2)
+__global__ void k_seg_recurrence(const double *__restrict__ vj, uint64_t n, const double *__restrict__ ab, uint32_t j,
+                                 uint32_t S, const uint32_t *__restrict__ sidx, double *__restrict__ w)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (j + 1) * S) return;
-    const uint32_t r = t / S, sg = t - r * S;
-    double v = 0.0;
-    if (r == j) v = ab[((size_t)j * 2) * S + sg];
-    else if (r + 1 == j) v = sqrt(ab[((size_t)r * 2 + 1) * S + sg]);
-    c[t] = v;
+    const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    const uint32_t sg = sidx[g];
+    double acc = 0.0;
+    if (j) acc += sqrt(ab[((size_t)j * 2 - 1) * S + sg]) * (vj - n)[g];
+    acc += ab[((size_t)j * 2) * S + sg] * vj[g];
+    w[g] -= acc;
 }
 
-// v_{j+1}[g] = w[g] / beta_j(s) while segment s still steps (j + 1 < its
-// step count and no breakdown so far), else 0
+// live[s]: segment s still steps after step j (j + 1 < its step count and no
+// breakdown so far)
+__global__ void k_seg_live(const double *__restrict__ ab, uint32_t j, uint32_t S, const uint32_t *__restrict__ iters,
+                           uint32_t *__restrict__ live)
+{
+    const uint32_t sg = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sg >= S) return;
+    live[sg] = (j == 0 || live[sg]) && j + 1 < iters[sg] && sqrt(ab[((size_t)j * 2 + 1) * S + sg]) >= 1e-12;
+}
+
+// v_{j+1}[g] = w[g] / beta_j(s) while segment s still steps, else 0
 __global__ void k_seg_next(const double *__restrict__ w, uint64_t n, const uint32_t *__restrict__ sidx,
-                           const double *__restrict__ ab, uint32_t j, uint32_t S, const uint32_t *__restrict__ iters,
+                           const double *__restrict__ ab, uint32_t j, uint32_t S, const uint32_t *__restrict__ live,
                            double *__restrict__ vnext)
 {
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t sg = sidx[g];
-    if (sg == ~0u) return;
-    bool live = j + 1 < iters[sg];
-    for (uint32_t r = 0; live && r <= j; r++) live = sqrt(ab[((size_t)r * 2 + 1) * S + sg]) >= 1e-12;
-    vnext[g] = live ? w[g] / sqrt(ab[((size_t)j * 2 + 1) * S + sg]) : 0.0;
+    vnext[g] = live[sg] ? w[g] / sqrt(ab[((size_t)j * 2 + 1) * S + sg]) : 0.0;
 }
 
-// start vectors: point g with local index l in component `label` gets the
-// same value k_random_start gives index l under seed + label; then scaled by
-// its segment's norm (sq = squared norms per segment)
-__global__ void k_seg_start(uint64_t n, const uint32_t *__restrict__ sidx, const uint32_t *__restrict__ lidx,
+// The tridiagonal problem of every segment, a block each: the steps up to the
+// first breakdown (m), their matrix from ab, cyclic Jacobi rotations in the
+// order of jacobi_eigen (the order fixes the eigenvectors' signs), and the
+// Ritz coefficients of the kk smallest eigenvalues, coef [kk][rows][S] (rows
+// beyond m zero, eigenvectors beyond found[s] unwritten). The rotation's
+// cosine and sine are formed from the half angle with two reciprocal square
+// roots, and entries below 1e-17 of the matrix's norm are left alone (the
+// sweeps end at 1e-15): both change it by rounding only. A chain of dependent
+// f64 operations bounds it, so the segments run side by side, threads 0-63 of
+// a block on the matrix and 64-127 on the vectors: 30 segments of 42 rows
+// 2.7 ms, 18 ms one after another on the host.
+__global__ void __launch_bounds__(128) k_seg_tridiag(const double *__restrict__ ab, uint32_t S, uint32_t rows, uint32_t kk,
+                                                    const uint32_t *__restrict__ iters, double *__restrict__ coef,
+                                                    uint32_t *__restrict__ found)
+{
+    extern __shared__ double sh[];
+    __shared__ double sums[2];
+    const uint32_t sg = blockIdx.x, tid = threadIdx.x, half = tid & 63;
+    const bool vectors = tid >= 64;
+    uint32_t m = iters[sg];
+    for (uint32_t r = 0; r < m; r++)
+        if (sqrt(fmax(0.0, ab[((size_t)r * 2 + 1) * S + sg])) < 1e-12) m = r + 1;
+    const uint32_t ld = rows | 1u;  // odd: a column's entries lie in different banks
+    double *A = sh, *V = sh + (size_t)rows * ld;  // V column k at V + k ld
+    for (uint32_t i = tid; i < m * ld; i += 128) A[i] = V[i] = 0.0;
+    __syncthreads();
+    for (uint32_t i = tid; i < m; i += 128) {
+        A[i * ld + i] = ab[((size_t)i * 2) * S + sg];
+        V[i * ld + i] = 1.0;
+        if (i + 1 < m) A[i * ld + i + 1] = A[(i + 1) * ld + i] = sqrt(fmax(0.0, ab[((size_t)i * 2 + 1) * S + sg]));
+    }
+    __syncthreads();
+    for (int sweep = 0; sweep < 100; sweep++) {
+        if (tid < 32) {
+            double off = 0.0, tot = 0.0;
+            for (uint32_t r = 0; r < m; r++)
+                for (uint32_t c = tid; c < m; c += 32) {
+                    const double x = A[r * ld + c];
+                    tot += x * x;
+                    if (r != c) off += x * x;
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                off += __shfl_xor_sync(0xFFFFFFFFu, off, o);
+                tot += __shfl_xor_sync(0xFFFFFFFFu, tot, o);
+            }
+            if (tid == 0) {
+                sums[0] = off;
+                sums[1] = tot;
+            }
+        }
+        __syncthreads();
+        const double off = sums[0], tot = sums[1];
+        if (off <= 1e-30 * (tot > 0.0 ? tot : 1.0)) break;
+        const double least = 1e-34 * tot;
+        for (uint32_t p = 0; p + 1 < m; p++)
+            for (uint32_t q = p + 1; q < m; q++) {
+                const double apq = A[p * ld + q];
+                if (fabs(apq) < 1e-300 || apq * apq < least) continue;  // block-uniform
+                // angle below 45 degrees with tan 2x = 2 apq / d; the sign of
+                // d / (2 apq), zero counting as positive
+                const double d = A[q * ld + q] - A[p * ld + p], h = 2.0 * fabs(apq);
+                const bool up = d == 0.0 || (d > 0.0) == (apq > 0.0);
+                const double ir = rsqrt(d * d + h * h), c2 = 0.5 + 0.5 * fabs(d) * ir, ic = rsqrt(c2);
+                const double c = c2 * ic, sa = 0.5 * h * ir * ic, s = up ? sa : -sa;
+                // symmetric update of rows and columns p, q; V := V J
+                double x[2], y[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const uint32_t k = half + 64 * i;
+                    if (k >= m) continue;
+                    x[i] = vectors ? V[p * ld + k] : A[p * ld + k];
+                    y[i] = vectors ? V[q * ld + k] : A[q * ld + k];
+                }
+                const double app = A[p * ld + p], aqq = A[q * ld + q], ta = s * ic * apq;
+                __syncthreads();  // every entry the rotation uses is read
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const uint32_t k = half + 64 * i;
+                    if (k >= m) continue;
+                    const double xn = c * x[i] - s * y[i], yn = s * x[i] + c * y[i];
+                    if (vectors) {
+                        V[p * ld + k] = xn;
+                        V[q * ld + k] = yn;
+                    } else if (k == p) {
+                        A[p * ld + p] = app - ta;
+                        A[p * ld + q] = A[q * ld + p] = 0.0;
+                    } else if (k == q) {
+                        A[q * ld + q] = aqq + ta;
+                    } else {
+                        A[p * ld + k] = A[k * ld + p] = xn;
+                        A[q * ld + k] = A[k * ld + q] = yn;
+                    }
+                }
+                __syncthreads();
+            }
+    }
+    const uint32_t have = min(kk, m);
+    if (tid == 0) found[sg] = have;
+    // the place of each eigenvalue in ascending order, equal ones by index; a
+    // warp each
+    for (uint32_t i = tid >> 5; i < m; i += 4) {
+        const double x = A[i * ld + i];
+        uint32_t e = 0;
+        for (uint32_t k = tid & 31; k < m; k += 32) {
+            const double y = A[k * ld + k];
+            e += (y < x || (y == x && k < i)) ? 1u : 0u;
+        }
+        e = __reduce_add_sync(0xFFFFFFFFu, e);
+        if (e < have)
+            for (uint32_t r = tid & 31; r < rows; r += 32) coef[((size_t)e * rows + r) * S + sg] = r < m ? V[i * ld + r] : 0.0;
+    }
+}
+
+// start vectors: member l of component `label` gets the same value
+// k_random_start gives index l under seed + label; then scaled by its
+// segment's norm (sq = squared norms per segment)
+__global__ void k_seg_start(uint64_t n, const uint32_t *__restrict__ sidx, const uint32_t *__restrict__ seg_beg,
                             const uint32_t *__restrict__ seg_label, uint64_t seed, double *__restrict__ v)
 {
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t sg = sidx[g];
-    if (sg == ~0u) {
-        v[g] = 0.0;
-        return;
-    }
-    uint64_t z = (seed + seg_label[sg]) + 0x9E3779B97F4A7C15ull * (uint64_t)(lidx[g] + 1);
+    uint64_t z = (seed + seg_label[sg]) + 0x9E3779B97F4A7C15ull * (g - seg_beg[sg] + 1);
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     z ^= z >> 31;
     v[g] = (double)(z >> 11) * (1.0 / 9007199254740992.0) - 0.5;
+}
+
+// The renumbering: point mem[i] becomes i, of the segment whose range
+// [seg_beg[s], seg_beg[s + 1]) holds i; rows[i] its number of entries.
+__global__ void k_seg_number(const uint32_t *__restrict__ mem, uint32_t n, const uint32_t *__restrict__ seg_beg, uint32_t S,
+                             const uint64_t *__restrict__ ptr, uint32_t *__restrict__ place, uint32_t *__restrict__ sidx,
+                             unsigned long long *__restrict__ rows)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t lo = 0, hi = S;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (seg_beg[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    const uint32_t g = mem[i];
+    sidx[i] = lo;
+    place[g] = i;
+    rows[i] = ptr[g + 1] - ptr[g];
+}
+
+// Row i of the renumbered matrix: row mem[i]'s entries in their order (all in
+// the same component, so every column has a place), eight lanes a row.
+__global__ void k_seg_rows(const uint32_t *__restrict__ mem, uint32_t n, const uint64_t *__restrict__ ptr,
+                           const uint32_t *__restrict__ col, const double *__restrict__ val,
+                           const uint32_t *__restrict__ place, const uint64_t *__restrict__ ptr2,
+                           uint32_t *__restrict__ col2, double *__restrict__ val2)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kRowLanes, lane = t % kRowLanes;
+    if (i >= n) return;
+    const uint64_t b = ptr[mem[i]], e = ptr[mem[i] + 1], to = ptr2[i];
+    for (uint64_t p = b + lane; p < e; p += kRowLanes) {
+        col2[to + (p - b)] = place[col[p]];
+        val2[to + (p - b)] = val[p];
+    }
 }
 
 __global__ void k_seg_scale(double *__restrict__ v, uint64_t n, const uint32_t *__restrict__ sidx,
@@ -423,7 +609,6 @@ __global__ void k_seg_scale(double *__restrict__ v, uint64_t n, const uint32_t *
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t sg = sidx[g];
-    if (sg == ~0u) return;
     const double nr = sqrt(sq[sg]);
     if (nr > 0.0) v[g] /= nr;
 }
@@ -431,15 +616,15 @@ __global__ void k_seg_scale(double *__restrict__ v, uint64_t n, const uint32_t *
 // -D^-1/2 A D^-1/2 of a COO graph on n nodes (graph_to_negative_normalised_
 // adjacency, src/data/init.rs:210-256) built on the device: degrees include
 // self loops, self-loop entries carry 0 (the reference drops them), CSR rows
-// keep the input order (stable sort by row). Host arrays in, device CSR out.
-void neg_normalised_adjacency(uint32_t n, uint64_t nnz, const uint32_t *row, const uint32_t *col, const float *w,
-                              DevBuf<uint64_t> &ptr, DevBuf<uint32_t> &cidx, DevBuf<double> &val, cudaStream_t s)
+// keep the input order (stable sort by row). Endpoints on the device, host
+// weights in, device CSR out.
+void neg_normalised_adjacency(uint32_t n, uint64_t nnz, const DevBuf<uint32_t> &drow, const DevBuf<uint32_t> &dcol,
+                              const float *w, DevBuf<uint64_t> &ptr, DevBuf<uint32_t> &cidx, DevBuf<double> &val,
+                              cudaStream_t s)
 {
     const uint64_t m = nnz ? nnz : 1;
-    DevBuf<uint32_t> drow(m, s), dcol(m, s), rs(m, s), perm0(m, s), perm(m, s);
+    DevBuf<uint32_t> rs(m, s), perm0(m, s), perm(m, s);
     DevBuf<float> dw(m, s);
-    h2d(drow.p, row, nnz, s);
-    h2d(dcol.p, col, nnz, s);
     h2d(dw.p, w, nnz, s);
     DevBuf<unsigned long long> cnt(n + 1, s);
     check_cuda(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long) * (n + 1), s), "memset");
@@ -502,13 +687,10 @@ __global__ void k_cc_jump(uint32_t *__restrict__ lab, uint32_t n)
     lab[i] = l;
 }
 
-void component_labels(uint32_t n, uint64_t nnz, const uint32_t *row, const uint32_t *col,
+void component_labels(uint32_t n, uint64_t nnz, const DevBuf<uint32_t> &drow, const DevBuf<uint32_t> &dcol,
                       std::vector<uint32_t> &labels, cudaStream_t s)
 {
-    const uint64_t m = nnz ? nnz : 1;
-    DevBuf<uint32_t> drow(m, s), dcol(m, s), lab(n, s), changed(1, s);
-    h2d(drow.p, row, nnz, s);
-    h2d(dcol.p, col, nnz, s);
+    DevBuf<uint32_t> lab(n, s), changed(1, s);
     k_iota<<<ceil_div(n, kBlk), kBlk, 0, s>>>(lab.p, n);
     for (uint32_t it = 0; nnz && it < 4096; it++) {
         uint32_t h = 0;
@@ -558,16 +740,16 @@ void batched_component_raw(uint32_t n, const DevBuf<uint64_t> &ptr, const DevBuf
     const uint32_t S = (uint32_t)solve.size();
     if (!S) return;
     const uint32_t kk = n_comp + 1;
-    std::vector<uint32_t> hmem, hsidx(n, ~0u), hlidx(n, 0), hlabel(S), hiters(S), hbeg, hend, hpofs(S + 1, 0);
+    std::vector<uint32_t> hmem, hseg(S + 1, 0), hlabel(S), hiters(S), hbeg, hend, hpofs(S + 1, 0);
+    size_t total = 0;
+    for (uint32_t q : solve) total += members[q].size();
+    hmem.reserve(total);
     uint32_t it_max = 0;
     for (uint32_t q = 0; q < S; q++) {
         const std::vector<uint32_t> &mem = members[solve[q]];
         const uint32_t at = (uint32_t)hmem.size();
-        for (uint32_t l = 0; l < mem.size(); l++) {
-            hsidx[mem[l]] = q;
-            hlidx[mem[l]] = l;
-            hmem.push_back(mem[l]);
-        }
+        hmem.insert(hmem.end(), mem.begin(), mem.end());
+        hseg[q + 1] = (uint32_t)hmem.size();
         for (uint32_t b = 0; b < mem.size(); b += kSegChunk) {
             hbeg.push_back(at + b);
             hend.push_back(at + std::min<uint32_t>(b + kSegChunk, (uint32_t)mem.size()));
@@ -577,86 +759,109 @@ void batched_component_raw(uint32_t n, const DevBuf<uint64_t> &ptr, const DevBuf
         hiters[q] = std::min<uint32_t>(kk * 4 + 30, (uint32_t)mem.size());
         it_max = std::max(it_max, hiters[q]);
     }
-    const uint32_t n_items = (uint32_t)hbeg.size();
-    DevBuf<uint32_t> mem(hmem.size(), s), ibeg(n_items, s), iend(n_items, s), pofs(S + 1, s), sidx(n, s), lidx(n, s),
-        label(S, s), iters(S, s);
-    h2d(mem.p, hmem.data(), hmem.size(), s);
+    const uint32_t n_items = (uint32_t)hbeg.size(), n_all = n;
+    n = (uint32_t)hmem.size();  // from here on: the solved components' points
+    DevBuf<uint32_t> mem(n, s), place(n_all, s), ibeg(n_items, s), iend(n_items, s), pofs(S + 1, s), sidx(n, s), seg(S + 1, s),
+        label(S, s), iters(S, s), live(S, s), dfound(S, s);
+    h2d(mem.p, hmem.data(), n, s);
     h2d(ibeg.p, hbeg.data(), n_items, s);
     h2d(iend.p, hend.data(), n_items, s);
     h2d(pofs.p, hpofs.data(), S + 1, s);
-    h2d(sidx.p, hsidx.data(), n, s);
-    h2d(lidx.p, hlidx.data(), n, s);
+    h2d(seg.p, hseg.data(), S + 1, s);
     h2d(label.p, hlabel.data(), S, s);
     h2d(iters.p, hiters.data(), S, s);
-    DevBuf<double> V((size_t)it_max * n, s), w(n, s), c((size_t)it_max * S, s), ab((size_t)it_max * 2 * S, s),
+    DevBuf<uint64_t> ptr2((size_t)n + 1, s);
+    DevBuf<uint32_t> ci2(ci.n, s);
+    DevBuf<double> val2(val.n, s);
+    {
+        DevBuf<unsigned long long> rows((size_t)n + 1, s);
+        check_cuda(cudaMemsetAsync(rows.p + n, 0, sizeof(unsigned long long), s), "memset");
+        k_seg_number<<<ceil_div(n, kBlk), kBlk, 0, s>>>(mem.p, n, seg.p, S, ptr.p, place.p, sidx.p, rows.p);
+        size_t tb = 0;
+        check_cuda(cub::DeviceScan::ExclusiveSum(nullptr, tb, rows.p, (unsigned long long *)ptr2.p, (int64_t)n + 1, s),
+                   "scan size");
+        DevBuf<char> tmp(tb ? tb : 1, s);
+        check_cuda(cub::DeviceScan::ExclusiveSum(tmp.p, tb, rows.p, (unsigned long long *)ptr2.p, (int64_t)n + 1, s),
+                   "scan");
+        k_seg_rows<<<ceil_div((uint64_t)n * kRowLanes, kBlk), kBlk, 0, s>>>(mem.p, n, ptr.p, ci.p, val.p, place.p, ptr2.p,
+                                                                            ci2.p, val2.p);
+        check_launch("renumbered matrix");
+    }
+    DevBuf<double> V((size_t)it_max * n, s), w(n, s), c((size_t)it_max * S * kk, s), ab((size_t)it_max * 2 * S, s),
         part((size_t)it_max * n_items, s), sq(S, s);
-    check_cuda(cudaMemsetAsync(V.p, 0, sizeof(double) * V.n, s), "memset");  // rows of unsolved points stay 0
+    check_cuda(cudaMemsetAsync(V.p, 0, sizeof(double) * V.n, s), "memset");
     const unsigned g = ceil_div(n, kBlk);
     auto seg_dots = [&](const double *Vrows, uint32_t rows, const double *x, double *out) {
-        k_seg_dots_part<<<dim3(n_items, rows), kBlk, 0, s>>>(Vrows, n, x, mem.p, ibeg.p, iend.p, n_items, part.p);
-        k_seg_sum_parts<<<ceil_div((uint64_t)rows * S, 128), 128, 0, s>>>(part.p, n_items, pofs.p, S, rows, out);
+        k_seg_dots_part<<<dim3(n_items, rows), kBlk, 0, s>>>(Vrows, n, x, ibeg.p, iend.p, n_items, part.p);
+        k_seg_sum_parts<<<ceil_div((uint64_t)rows * S * 32, 128), 128, 0, s>>>(part.p, n_items, pofs.p, S, rows, out);
     };
-    k_seg_start<<<g, kBlk, 0, s>>>(n, sidx.p, lidx.p, label.p, seed, V.p);
+    k_seg_start<<<g, kBlk, 0, s>>>(n, sidx.p, seg.p, label.p, seed, V.p);
     seg_dots(V.p, 1, V.p, sq.p);
     k_seg_scale<<<g, kBlk, 0, s>>>(V.p, n, sidx.p, sq.p);
     check_launch("batched start");
     for (uint32_t j = 0; j < it_max; j++) {
         const double *vj = V.p + (size_t)j * n;
-        k_spmv<<<ceil_div((uint64_t)n * 32, kBlk), kBlk, 0, s>>>(n, ptr.p, ci.p, val.p, vj, w.p);
+        k_spmv<<<ceil_div((uint64_t)n * kRowLanes, kBlk), kBlk, 0, s>>>(n, ptr2.p, ci2.p, val2.p, vj, w.p);
         seg_dots(vj, 1, w.p, ab.p + (size_t)j * 2 * S);  // alpha_j per segment
-        k_seg_recurrence<<<ceil_div((uint64_t)(j + 1) * S, 128), 128, 0, s>>>(ab.p, j, S, c.p);
-        k_seg_comb<<<g, kBlk, 0, s>>>(V.p, n, j + 1, c.p, S, sidx.p, w.p, true);
+        k_seg_recurrence<<<g, kBlk, 0, s>>>(vj, n, ab.p, j, S, sidx.p, w.p);
         for (int pass = 0; pass < 2; pass++) {
             seg_dots(V.p, j + 1, w.p, c.p);
             k_seg_comb<<<g, kBlk, 0, s>>>(V.p, n, j + 1, c.p, S, sidx.p, w.p, true);
         }
         seg_dots(w.p, 1, w.p, ab.p + ((size_t)j * 2 + 1) * S);  // beta_j^2
-        if (j + 1 < it_max)
-            k_seg_next<<<g, kBlk, 0, s>>>(w.p, n, sidx.p, ab.p, j, S, iters.p, V.p + (size_t)(j + 1) * n);
+        if (j + 1 < it_max) {
+            k_seg_live<<<ceil_div(S, 128), 128, 0, s>>>(ab.p, j, S, iters.p, live.p);
+            k_seg_next<<<g, kBlk, 0, s>>>(w.p, n, sidx.p, ab.p, j, S, live.p, V.p + (size_t)(j + 1) * n);
+        }
         check_launch("batched lanczos step");
     }
-    std::vector<double> hab((size_t)it_max * 2 * S);
-    d2h(hab.data(), ab.p, hab.size(), s);
-    sync(s);
-    // per component: truncate, tridiagonal eigenproblem; keep the Ritz
-    // coefficients of its kk smallest eigenvalues (ritz[q] [e][m_q])
-    std::vector<std::vector<double>> ritz(S);
-    std::vector<uint32_t> found(S), msteps(S);
-    for (uint32_t q = 0; q < S; q++) {
-        std::vector<double> alpha, beta;
-        for (uint32_t j = 0; j < hiters[q]; j++) {
-            alpha.push_back(hab[((size_t)j * 2) * S + q]);
-            beta.push_back(std::sqrt(std::max(0.0, hab[((size_t)j * 2 + 1) * S + q])));
-            if (beta.back() < 1e-12) break;
+    // per component: truncate, tridiagonal eigenproblem; the Ritz coefficients
+    // of its kk smallest eigenvalues, c [kk][it_max][S]. On the device for
+    // several components of up to kTridiagRows rows (both matrices in shared
+    // memory); a single one is as fast on the host.
+    std::vector<uint32_t> found(S);
+    constexpr uint32_t kTridiagRows = 110;
+    if (S > 1 && it_max <= kTridiagRows) {
+        const size_t smem = 2 * sizeof(double) * it_max * (it_max | 1u);
+        check_cuda(cudaFuncSetAttribute(k_seg_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                   "tridiagonal shared memory");
+        k_seg_tridiag<<<S, 128, smem, s>>>(ab.p, S, it_max, kk, iters.p, c.p, dfound.p);
+        check_launch("k_seg_tridiag");
+        d2h(found.data(), dfound.p, S, s);
+        sync(s);
+    } else {
+        std::vector<double> hab((size_t)it_max * 2 * S), coef((size_t)kk * it_max * S, 0.0);
+        d2h(hab.data(), ab.p, hab.size(), s);
+        sync(s);
+        for (uint32_t q = 0; q < S; q++) {
+            std::vector<double> alpha, beta;
+            for (uint32_t j = 0; j < hiters[q]; j++) {
+                alpha.push_back(hab[((size_t)j * 2) * S + q]);
+                beta.push_back(std::sqrt(std::max(0.0, hab[((size_t)j * 2 + 1) * S + q])));
+                if (beta.back() < 1e-12) break;
+            }
+            const uint32_t m = (uint32_t)alpha.size();
+            std::vector<double> T((size_t)m * m, 0.0), tev, tvec;
+            for (uint32_t i = 0; i < m; i++) {
+                T[(size_t)i * m + i] = alpha[i];
+                if (i + 1 < m) T[(size_t)i * m + i + 1] = T[(size_t)(i + 1) * m + i] = beta[i];
+            }
+            jacobi_eigen(T, m, tev, tvec);
+            std::vector<uint32_t> order(m);
+            std::iota(order.begin(), order.end(), 0u);
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return tev[x] < tev[y]; });
+            found[q] = std::min(kk, m);
+            for (uint32_t e = 0; e < found[q]; e++)
+                for (uint32_t r = 0; r < m; r++) coef[((size_t)e * it_max + r) * S + q] = tvec[(size_t)order[e] * m + r];
         }
-        const uint32_t m = (uint32_t)alpha.size();
-        std::vector<double> T((size_t)m * m, 0.0), tev, tvec;
-        for (uint32_t i = 0; i < m; i++) {
-            T[(size_t)i * m + i] = alpha[i];
-            if (i + 1 < m) T[(size_t)i * m + i + 1] = T[(size_t)(i + 1) * m + i] = beta[i];
-        }
-        jacobi_eigen(T, m, tev, tvec);
-        std::vector<uint32_t> order(m);
-        std::iota(order.begin(), order.end(), 0u);
-        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return tev[x] < tev[y]; });
-        found[q] = std::min(kk, m);
-        msteps[q] = m;
-        ritz[q].resize((size_t)found[q] * m);
-        for (uint32_t e = 0; e < found[q]; e++)
-            std::copy(tvec.begin() + (size_t)order[e] * m, tvec.begin() + (size_t)(order[e] + 1) * m,
-                      ritz[q].begin() + (size_t)e * m);
+        h2d(c.p, coef.data(), coef.size(), s);
+        sync(s);
     }
     // back-transform eigenvector e of every component, normalise per component
     for (uint32_t q = 0; q < S; q++) raw[solve[q]].assign(members[solve[q]].size() * n_comp, 0.0);
-    std::vector<double> hv(n), hn(S), coef((size_t)it_max * S);
+    std::vector<double> hv(n), hn(S);
     for (uint32_t e = 1; e < kk; e++) {
-        std::fill(coef.begin(), coef.end(), 0.0);  // [r][s]
-        for (uint32_t q = 0; q < S; q++)
-            if (e < found[q])
-                for (uint32_t r = 0; r < msteps[q]; r++)
-                    coef[(size_t)r * S + q] = ritz[q][(size_t)e * msteps[q] + r];
-        h2d(c.p, coef.data(), coef.size(), s);
-        k_seg_comb<<<g, kBlk, 0, s>>>(V.p, n, it_max, c.p, S, sidx.p, w.p, false);
+        k_seg_comb<<<g, kBlk, 0, s>>>(V.p, n, it_max, c.p + (size_t)e * it_max * S, S, sidx.p, w.p, false);
         seg_dots(w.p, 1, w.p, sq.p);
         check_launch("batched back-transform");
         d2h(hv.data(), w.p, n, s);
@@ -669,7 +874,7 @@ void batched_component_raw(uint32_t n, const DevBuf<uint64_t> &ptr, const DevBuf
             if (e < found[q]) {
                 const double nr = std::sqrt(hn[q]);
                 for (uint32_t l = 0; l < mem.size(); l++)
-                    out[(size_t)l * n_comp + d] = (double)(float)(nr > 0 ? hv[mem[l]] / nr : hv[mem[l]]);
+                    out[(size_t)l * n_comp + d] = (double)(float)(nr > 0 ? hv[hseg[q] + l] / nr : hv[hseg[q] + l]);
             } else {
                 Mix r{seed + solve[q] + d};
                 for (uint32_t l = 0; l < mem.size(); l++) out[(size_t)l * n_comp + d] = 2.0 * r.uniform() - 1.0;
@@ -781,7 +986,10 @@ umapcu_status umapcu_spectral_layout(const uint32_t *row, const uint32_t *col, c
         // connected components (find_connected_components, init.rs:349-391),
         // labelled in order of their smallest point, members ascending
         std::vector<uint32_t> root;
-        component_labels(n, nnz, row, col, root, st.s);
+        DevBuf<uint32_t> drow(nnz ? nnz : 1, st.s), dcol(nnz ? nnz : 1, st.s);
+        h2d(drow.p, row, nnz, st.s);
+        h2d(dcol.p, col, nnz, st.s);
+        component_labels(n, nnz, drow, dcol, root, st.s);
         lap("components");
         std::vector<uint32_t> cid(n, ~0u);
         std::vector<std::vector<uint32_t>> members;
@@ -804,7 +1012,7 @@ umapcu_status umapcu_spectral_layout(const uint32_t *row, const uint32_t *col, c
                 DevBuf<uint64_t> ptr;
                 DevBuf<uint32_t> ci;
                 DevBuf<double> av;
-                neg_normalised_adjacency(n, nnz, row, col, val, ptr, ci, av, st.s);
+                neg_normalised_adjacency(n, nnz, drow, dcol, val, ptr, ci, av, st.s);
                 std::vector<std::vector<double>> raw(1);
                 batched_component_raw(n, ptr, ci, av, members, {0u}, n_comp, seed, raw, st.s);
                 out.swap(raw[0]);
@@ -849,7 +1057,7 @@ umapcu_status umapcu_spectral_layout(const uint32_t *row, const uint32_t *col, c
                 DevBuf<uint64_t> ptr;
                 DevBuf<uint32_t> ci;
                 DevBuf<double> av;
-                neg_normalised_adjacency(n, nnz, row, col, val, ptr, ci, av, st.s);
+                neg_normalised_adjacency(n, nnz, drow, dcol, val, ptr, ci, av, st.s);
                 for (size_t b = 0; b < solve.size(); b += 16384) {
                     const std::vector<uint32_t> part(solve.begin() + b,
                                                      solve.begin() + std::min(solve.size(), b + 16384));

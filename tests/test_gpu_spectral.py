@@ -159,3 +159,29 @@ def test_spectral_layout_components_solved_together_match_oracle():
             corr = np.corrcoef(V[:, 1 + d], y[sl, d])[0, 1]
             assert abs(corr) > 0.9999, (label, d, corr)
         off += m
+
+
+@pytest.mark.parametrize("n_comp,sizes", [(2, (40, 45, 300, 2100)), (5, (60, 700)), (20, (150, 260))])
+def test_spectral_layout_tridiagonal_forms(n_comp, sizes):
+    """Components solved together with step counts below, at and above what
+    the device's tridiagonal solver holds (n_comp = 20: 114 rows, solved on the
+    host): each component's coordinates along its leading eigenvectors against
+    the oracle's Lanczos of that component alone."""
+    from oracle import oracle as O
+    parts, off = [], 0
+    for i, m in enumerate(sizes):
+        g = _strip_graph(m, seed=31 + i)
+        parts.append((g["row"] + off, g["col"] + off, g["val"]))
+        off += m
+    r, c, v = (np.concatenate([p[k] for p in parts]) for k in range(3))
+    coo = umapcu.CoordinateList(r.astype(np.uint32), c.astype(np.uint32), v.astype(np.float32), off)
+    y = umapcu.spectral_layout(coo, n_comp, seed=9)
+    assert y.shape == (off, n_comp) and np.isfinite(y).all()
+    off = 0
+    for label, m in enumerate(sizes):
+        sub = dict(row=parts[label][0] - off, col=parts[label][1] - off, val=parts[label][2])
+        _, V = O.lanczos_smallest(_neg_norm_adjacency(sub, m), n_comp + 1, O.splitmix_start(m, 9 + label))
+        for d in range(2):  # the modes along the strip, well separated
+            corr = np.corrcoef(V[:, 1 + d], y[off:off + m, d])[0, 1]
+            assert abs(corr) > 0.9999, (label, d, corr)
+        off += m
