@@ -447,8 +447,9 @@ umapcu_status umapcu_state_schedule_form(const umapcu_state *st, uint32_t *form)
  * default): raise them again on the next call. */
 umapcu_status umapcu_set_pool_retention(int keep);
 
-/* Frees the current device's cached bitmask block and trims its default
- * pool to the memory in use. */
+/* Frees the current device's cached bitmask block and the process's
+ * page-locked copy block, and trims the device's default pool to the memory in
+ * use. */
 umapcu_status umapcu_release_cached(void);
 
 /* Devices (no counterpart in the reference, which takes one device per

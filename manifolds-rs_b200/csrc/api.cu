@@ -995,6 +995,7 @@ umapcu_status umapcu_release_cached(void)
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return UMAPCU_NO_DEVICE;
         release_cached_bits();
+        release_copy_block();
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
         return UMAPCU_OK;

@@ -115,14 +115,22 @@ struct Event {
     void record(cudaStream_t s) { check_cuda(cudaEventRecord(e, s), "cudaEventRecord"); }
 };
 
+// A large copy between pageable host memory and the device by several threads
+// (hostcopy.cu), finished when it returns; false: not such a copy, nothing done.
+bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaStream_t s);
+// Frees the page-locked block such copies go through, unless one is under way.
+void release_copy_block();
+
 template <typename T>
 inline void h2d(T *dst, const T *src, size_t count, cudaStream_t s)
 {
+    if (staged_copy(dst, src, count * sizeof(T), true, s)) return;
     if (count) check_cuda(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyHostToDevice, s), "h2d");
 }
 template <typename T>
 inline void d2h(T *dst, const T *src, size_t count, cudaStream_t s)
 {
+    if (staged_copy(dst, src, count * sizeof(T), false, s)) return;
     if (count) check_cuda(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, s), "d2h");
 }
 inline void sync(cudaStream_t s) { check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize"); }

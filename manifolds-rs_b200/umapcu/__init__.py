@@ -322,8 +322,9 @@ def construct_umap_graph(knn_indices, knn_dists, umap_params: UmapGraphParams = 
     cg = _GraphParams(gp.bandwidth, gp.local_connectivity, gp.mix_weight)
     _check(_lib.umapcu_construct_umap_graph(_p(idx), _p(d), n, k, C.byref(cg), n_epochs, cap, _p(row), _p(col),
                                             _p(val), C.byref(nnz), _p(sig), _p(rho)))
-    m = nnz.value
-    g = CoordinateList(row[:m].copy(), col[:m].copy(), val[:m].copy(), n)
+    for a in (row, col, val):  # give back what the graph does not fill, without a copy
+        a.resize(nnz.value, refcheck=False)
+    g = CoordinateList(row, col, val, n)
     return (g, sig, rho) if return_sigma_rho else g
 
 
@@ -778,8 +779,9 @@ def set_pool_retention(keep: bool = True):
 
 
 def release_cached():
-    """Frees the current device's cached schedule-bitmask block and trims its
-    default memory pool."""
+    """Frees the current device's cached schedule-bitmask block and the
+    process's page-locked copy block, and trims the device's default memory
+    pool."""
     _check(_lib.umapcu_release_cached(), "release_cached")
 
 
