@@ -59,7 +59,7 @@ template <int EPI>
 struct __align__(16) TileSmem {
     float q[2][kDC][kQS];
     float p[2][kDC][kPS];
-    uint32_t qrow[kQT];
+    uint32_t qrow[kQT], qpos[kQT];  // the queries' rows, and their places among all queries
     // EPI_RANK: each query's thresholds ascending, which of the given ones
     // each is, and the points counted per sorted threshold
     float thr[EPI == EPI_RANK ? kQT : 1][32];
@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
     if (tid < kQT) {
         const uint32_t q = q0 + tid < nq ? (A.left ? A.left[q0 + tid] : q0 + tid) : 0u;
         S.qrow[tid] = q0 + tid < nq ? (A.qidx ? A.qidx[q] : q) : 0u;
+        S.qpos[tid] = q;
     }
     __syncthreads();
 
@@ -195,8 +196,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
             float td = __int_as_float(0x7fffffff);
             uint32_t tj = ~0u;
             if (lane < A.k) {
-                td = A.thr_d[(size_t)(q0 + ql) * A.k + lane];
-                tj = A.thr_j[(size_t)(q0 + ql) * A.k + lane];
+                td = A.thr_d[(size_t)S.qpos[ql] * A.k + lane];
+                tj = A.thr_j[(size_t)S.qpos[ql] * A.k + lane];
             }
             uint32_t at = 0;  // a repeated neighbour keeps the order of the lanes
             for (uint32_t m = 0; m < A.k; m++) {
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
                     while (lo < hi) {
                         const uint32_t mid = (lo + hi) >> 1;
                         const float t = S.thr[ql][mid];
-                        const bool before = dv[j] < t || (dv[j] == t && pidx[j] < A.thr_j[(size_t)(q0 + ql) * A.k + S.given[ql][mid]]);
+                        const bool before = dv[j] < t || (dv[j] == t && pidx[j] < A.thr_j[(size_t)S.qpos[ql] * A.k + S.given[ql][mid]]);
                         if (before) hi = mid;
                         else lo = mid + 1;
                     }
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
         if (EPI == EPI_TOPK) {
             if (lane >= A.k) continue;
             // one slice writes the final place, several the merge's input
-            const size_t at = A.left && gridDim.y == 1 ? A.left[q] : q;
+            const size_t at = gridDim.y == 1 ? S.qpos[warp * 8 + i] : q;
             const size_t o = ((size_t)slice * A.nq + at) * A.k + lane;
             A.out_idx[o] = li[i];
             A.out_dist[o] = ld[i];
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_knn_tile(const TileArgs A)
                 if ((int)lane >= off) c += u;
             }
             const uint32_t mine = __shfl_sync(kFull, c, place[i] & 31u);
-            if (lane < A.k && place[i] != ~0u && mine) atomicAdd(&A.counts[q * A.k + lane], mine);
+            if (lane < A.k && place[i] != ~0u && mine) atomicAdd(&A.counts[(size_t)S.qpos[warp * 8 + i] * A.k + lane], mine);
         }
     }
 }
@@ -555,6 +556,18 @@ void knn_rank_dev(const float *d_x, uint32_t n, uint32_t dim, const uint32_t *d_
     A.qidx = d_qidx;
     A.nq = nq;
     A.tiles_per_slice = ceil_div(n_tiles, S);
+    // as in knn_dev: the filter, and the tile kernel for what it leaves
+    DevBuf<uint32_t> left, n_left;
+    if (rank_filter_takes(n, dim, nq, k)) {
+        left.alloc(nq, s);
+        n_left.alloc(1, s);
+        check_cuda(cudaMemsetAsync(n_left.p, 0, sizeof(uint32_t), s), "memset");
+        const KnnFilterArgs F{x, n, dim, k, euc, d_qidx, nq, nullptr, nullptr};
+        if (rank_filter(F, thr.p, d_nbr, d_counts, left.p, n_left.p, s)) {
+            A.left = left.p;
+            A.n_left = n_left.p;
+        }
+    }
     A.thr_d = thr.p;
     A.thr_j = d_nbr;
     A.counts = d_counts;

@@ -34,16 +34,29 @@
 // staging; two epilogue warps a scheduler instead of four, descriptors formed
 // in the loop and one lane issuing took 2.4 us. Against the FP32 tile kernel,
 // whole knn_exact calls: 10k x 50 dims, k = 15 1.81 -> 0.71 ms, 200k x 30 dims,
-// k = 30 166 -> 20.8 ms (of which the copies of host arrays take about 10).
+// k = 30 166 -> 15.6 ms (of which the copies of host arrays take about 5).
 //
-// Error bound. With u = |q|, v = |p|: the split leaves at most
-// 3.1 * 2^-16 u v (two pieces) or 2^-21 u v (six products) of a dot product,
-// f32 accumulation over at most 36 steps of 16 products 1e-5 (u v + v^2 / 2),
-// centring and norms a few 2^-24 of (u + v)^2; in all |s - s_true| <=
-// kappa (u^2 + v^2) with kappa as in filter_kappa, which is rounded up. The
-// chain distance itself is within (dim + 8) 2^-24 of the true one,
-// relatively. k_filter_threshold carries both, so no true neighbour is left
-// out; a looser threshold only means more candidates.
+// Ranks (trustworthiness: how many points are better than each of k given
+// neighbours of a query) use the same scores. k_rank_bounds turns the
+// neighbours' exact distances, sorted, into scores at or above which a point is
+// surely better (hi) and below which it surely is not (lo); k_filter<1, 3>
+// counts, per query, the points of every zone between them, and lists those
+// inside a [lo, hi) interval; k_rank_refine settles these by their exact
+// distances and adds up. 10k queries x 100k points x 50 dims, k = 15, whole
+// call: 15.1 -> 5.4 ms.
+//
+// Error bound. With u = |q|, v = |p|: of a dot product the contraction leaves
+// out lo.lo and the products with what the pieces leave of a coordinate; as
+// norms these are at most rho_l and rho_r of a row's, the largest of the data
+// (k_filter_norms), together u v (rho_l^2 + 2 rho_r + rho_r^2). (bf16 rounding
+// alone bounds that by 4.7e-5 u v for two pieces; random data have 7e-6, and a
+// seventh of the candidates near a threshold.) An MMA step adds 16 products to
+// the f32 accumulator, each cut to the largest's last place at worst: 2^-19.8 of
+// the magnitudes a step. Centring and norms: a few 2^-24 of (u + v)^2. In all
+// |s - s_true| <= kappa (u^2 + v^2) with filter_kappa. The chain distance
+// itself is within (dim + 8) 2^-24 of the true one, relatively.
+// k_filter_threshold carries both, so no true neighbour is left out; a looser
+// threshold only means more candidates.
 #include <cuda_bf16.h>
 
 #include <cfloat>
@@ -85,7 +98,13 @@ Pack pack_of(uint32_t dim)
     return p;
 }
 
-double filter_kappa(uint32_t terms) { return terms == 6 ? 4e-6 : 5e-5; }
+// kappa (above) of rows whose left-out parts are rho[0] (second pieces, when
+// their product is left out) and rho[1] (what all pieces leave) of their norms.
+__device__ __forceinline__ double filter_kappa(const float *rho, uint32_t steps)
+{
+    const double l = rho[0], r = rho[1];
+    return 0.52 * (l * l + 2.0 * r + r * r) + 1.1e-6 * steps + 0x1p-21;
+}
 
 // ------------------------------------------------------------ preparation
 
@@ -111,26 +130,6 @@ __global__ void __launch_bounds__(1024) k_filter_centre(const float *__restrict_
     if (g == 0 && d < dim) mu[d] = sh[0][e];
 }
 
-// |row - mu|^2 of every point, a warp per row; *bad set when a row is not
-// finite or its norm is beyond what the bound's arithmetic can hold.
-__global__ void k_filter_norms(const float *__restrict__ x, uint32_t n, uint32_t dim, const float *__restrict__ mu,
-                               float *__restrict__ norm, uint32_t *__restrict__ bad)
-{
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    double acc = 0.0;
-    for (uint32_t d = lane; d < dim; d += 32) {
-        const double v = (double)(x[(size_t)row * dim + d] - (mu ? mu[d] : 0.0f));
-        acc += v * v;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(kFull, acc, o);
-    if (lane == 0) {
-        norm[row] = (float)acc;
-        if (!(acc < 1e28)) *bad = 1u;
-    }
-}
-
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 // Piece t of v: what the t pieces before it leave, rounded to bf16.
@@ -142,6 +141,45 @@ __device__ __forceinline__ float bf16_piece(float v, uint32_t t)
         p = bf16_round(v);
     }
     return p;
+}
+
+// |row - mu|^2 of every point, a warp per row, and into rho the largest shares
+// of a row's norm that the contraction leaves out (filter_kappa); *bad set when
+// a row is not finite or its norm is beyond what the bound's arithmetic can
+// hold.
+__global__ void k_filter_norms(const float *__restrict__ x, uint32_t n, uint32_t dim, const float *__restrict__ mu,
+                               uint32_t terms, float *__restrict__ norm, float *__restrict__ rho,
+                               uint32_t *__restrict__ bad)
+{
+    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= n) return;
+    double acc = 0.0;
+    float second = 0.0f, rest = 0.0f;
+    for (uint32_t d = lane; d < dim; d += 32) {
+        const float f = x[(size_t)row * dim + d] - (mu ? mu[d] : 0.0f);
+        acc += (double)f * (double)f;
+        float r = f - bf16_round(f);
+        const float l = bf16_round(r);
+        r = r - l;
+        if (terms == 6) r = r - bf16_round(r);
+        else second += l * l;
+        rest += r * r;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        acc += __shfl_down_sync(kFull, acc, o);
+        second += __shfl_down_sync(kFull, second, o);
+        rest += __shfl_down_sync(kFull, rest, o);
+    }
+    if (lane != 0) return;
+    norm[row] = (float)acc;
+    if (!(acc < 1e28)) *bad = 1u;
+    if (!(acc > 1e-30)) return;  // (the bound's absolute part covers rows this small)
+    // (sums of up to 191 f32 squares: rounded up by 1e-4)
+    const float inv = (float)(1.0001 / acc);
+    const float a = sqrtf(second * inv), b = sqrtf(rest * inv);
+    if (a > rho[0]) atomicMax((int *)&rho[0], __float_as_int(a));  // (stale reads only cost an atomic)
+    if (b > rho[1]) atomicMax((int *)&rho[1], __float_as_int(b));
 }
 
 // The operands as the shared-memory images the MMA reads: K-major rows of 64
@@ -299,6 +337,12 @@ struct FilterArgs {
     uint32_t *list;          // [parts][nq][cap]
     uint32_t *count;         // [parts][nq], may exceed cap
     uint32_t cap;
+    // PASS 3 (list, count, cap as above)
+    uint32_t k, zone_rows;   // zone_rows = 2^steps - 1 >= k
+    const float *hi, *lo;    // [nq][k], descending
+    const uint32_t *qidx;    // the query rows, or nullptr: q0 + q
+    uint32_t q0;
+    uint32_t *zones;         // [nq][32], added to
     uint32_t *bad;           // set when a wait gave up
 };
 
@@ -312,7 +356,11 @@ struct FilterArgs {
 // MB = 1, for operands of more than three chunks, whose A would not leave room
 // for the ring: the accumulators alternate between tiles. 512 columns of TMEM
 // and more than half the shared memory: one block an SM.
-template <int MB, int PASS>
+// PASS 3 (MB = 1): per score a search of the query's hi scores in shared memory
+// (laid out by row, so that the lanes of a warp never meet in a bank), one
+// comparison with a lo score and one add to the thread's own zone counter; the
+// search bounds it. STEPS: of that search, 2^STEPS > k.
+template <int MB, int PASS, int STEPS = 0>
 __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P)
 {
     extern __shared__ uint8_t dyn[];
@@ -465,7 +513,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
                 for (int j = 0; j < 8; j++)
                     o[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
             }
-        } else {
+        } else if constexpr (PASS == 2) {
             const uint32_t part = (MB == 2 ? slice : slice * 2 + b) * 2 + half;
             const float least = q < P.nq ? P.least[q] : __int_as_float(0x7f800000);
             uint32_t *list = P.list + ((size_t)part * P.nq + (q < P.nq ? q : 0)) * P.cap;
@@ -521,6 +569,81 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
                     }
             }
             if (q < P.nq) P.count[(size_t)part * P.nq + q] = count;
+        } else {
+            const uint32_t part = (slice * 2 + b) * 2 + half;
+            float *tables = reinterpret_cast<float *>(sb + (size_t)R * kBBytes);
+            float *hi = tables + quarter * 32 + lane;         // [zone_rows][128]
+            float *lo = hi + (size_t)P.zone_rows * kBlkM;     // [k + 1][128]: row m of threshold m - 1, row 0 infinite
+            uint32_t *zone = reinterpret_cast<uint32_t *>(tables + (size_t)(P.zone_rows + P.k + 1) * kBlkM) + threadIdx.x;
+            const bool in = q < P.nq;
+            if (b == 0 && half == 0) {
+                for (uint32_t m = 0; m < P.zone_rows; m++)
+                    hi[m * kBlkM] = in && m < P.k ? P.hi[(size_t)q * P.k + m] : __int_as_float(0xff800000);
+                lo[0] = __int_as_float(0x7f800000);
+                for (uint32_t m = 0; m < P.k; m++)
+                    lo[(m + 1) * kBlkM] = in ? P.lo[(size_t)q * P.k + m] : __int_as_float(0x7f800000);
+            }
+            for (uint32_t m = 0; m <= P.k; m++) zone[m * 512] = 0;
+            asm volatile("bar.sync 1, 512;" ::: "memory");  // the epilogue warps
+            const uint32_t self = !in ? ~0u : P.qidx ? P.qidx[P.q0 + q] : P.q0 + q;
+            uint32_t *list = P.list + ((size_t)part * P.nq + (in ? q : 0)) * P.cap;
+            uint32_t count = 0;
+            for (uint32_t u = 0; ok && u < uses; u++) {
+                ok = __all_sync(kFull, bar_wait(&tfull[b], u & 1, stop));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t p0 = (slice + (2 * u + b) * P.slices) * P.stride * kTileN + half * kHalf;
+                for (int h = 0; h < (int)kHalf / 32; h++) {
+                    float w[32];
+                    tmem_ld32(t0 + 32 * h, w);
+                    tmem_wait(w);
+                    if (h + 1 == (int)kHalf / 32) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(&tempty[b]);
+                    }
+                    const uint32_t pc = p0 + 32 * h;
+                    if (self - pc < 32u) {  // the query itself counts for nothing
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (self - pc == (uint32_t)j) w[j] = __int_as_float(0xff800000);
+                    }
+                    uint32_t open = 0;
+#pragma unroll
+                    for (int j0 = 0; j0 < 32; j0 += 8) {
+                        // m: thresholds with hi above the score, which is
+                        // surely better than the later ones. Eight searches
+                        // side by side, and only then the counters: a store
+                        // between them would hold back the next one's loads
+                        uint32_t m[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) m[j] = 0;
+#pragma unroll
+                        for (int st = STEPS > 0 ? 1 << (STEPS - 1) : 0; st > 0; st >>= 1)
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
+                                if (w[j0 + j] < hi[(m[j] + st - 1) * kBlkM]) m[j] += st;
+                        // unsettled unless surely worse than the last of these
+                        uint32_t un = 0;
+#pragma unroll
+                        for (int j = 0; j < 8; j++) un |= w[j0 + j] >= lo[m[j] * kBlkM] ? 1u << j : 0u;
+                        open |= un << j0;
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                            if (!((un >> j) & 1u)) atomicAdd(&zone[m[j] * 512], 1u);
+                    }
+                    while (open) {
+                        if (count < P.cap) list[count] = pc + (uint32_t)__ffs(open) - 1u;
+                        count++;
+                        open &= open - 1u;
+                    }
+                }
+            }
+            if (in) {
+                P.count[(size_t)part * P.nq + q] = count;
+                for (uint32_t m = 0; m < P.k; m++)
+                    if (zone[m * 512]) atomicAdd(&P.zones[(size_t)q * 32 + m], zone[m * 512]);
+            }
         }
         if (!ok && lane == 0) *P.bad = 1u;
     }
@@ -544,7 +667,8 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
 // that of 1 - dot.
 __global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t parts, uint32_t nq, uint32_t k,
                                    const float *__restrict__ norm, const uint32_t *__restrict__ qidx, uint32_t q0,
-                                   uint32_t dim, bool euc, double kappa, float *__restrict__ least)
+                                   uint32_t dim, bool euc, const float *__restrict__ rho, uint32_t steps,
+                                   float *__restrict__ least)
 {
     const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (q >= nq) return;  // warp-uniform
@@ -569,6 +693,7 @@ __global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t part
         }
     }
     if (lane != 0) return;
+    const double kappa = filter_kappa(rho, steps);
     const double s = (double)__uint_as_float((top & 0x80000000u) ? top ^ 0x80000000u : ~top);
     double g;
     if (euc) {
@@ -589,12 +714,49 @@ __device__ __forceinline__ bool better(float d, uint32_t i, float td, uint32_t t
     return d < td || (d == td && i < ti);
 }
 
+// The chain distances (knn.cu) of a query's row xq to the 32 candidate rows
+// `mine`, one per lane, the first `rows` of them wanted: rows staged through
+// the warp's shared memory 32 dims at a time (coalesced; a lane reading its own
+// candidate's row would touch 32 lines a load).
+template <bool EUC>
+__device__ __forceinline__ float chain_distance(const float *__restrict__ x, uint32_t dim, const float *__restrict__ xq,
+                                                uint32_t mine, uint32_t rows, float (&S)[32][33], uint32_t lane)
+{
+    float acc = 0.0f;
+    for (uint32_t d0 = 0; d0 < dim; d0 += 32) {
+        const uint32_t w = min(32u, dim - d0);
+        __syncwarp();
+        if (w > 16) {
+#pragma unroll 8
+            for (uint32_t r = 0; r < rows; r++) {
+                const uint32_t id = __shfl_sync(kFull, mine, r);
+                if (lane < w) S[r][lane] = __ldg(x + (size_t)id * dim + d0 + lane);
+            }
+        } else {  // two rows a step
+            for (uint32_t r = 0; r < rows; r += 2) {
+                const uint32_t id = __shfl_sync(kFull, mine, (r + (lane >> 4)) & 31u);
+                const uint32_t e = lane & 15;
+                if (e < w) S[r + (lane >> 4)][e] = __ldg(x + (size_t)id * dim + d0 + e);
+            }
+        }
+        __syncwarp();
+        for (uint32_t d = 0; d < w; d++) {
+            const float a = __ldg(xq + d0 + d), v = S[lane][d];
+            if (EUC) {
+                const float df = a - v;
+                acc = __fmaf_rn(df, df, acc);
+            } else {
+                acc = __fmaf_rn(a, v, acc);
+            }
+        }
+    }
+    return EUC ? acc : 1.0f - acc;
+}
+
 // The exact second look, a warp per query: 32 candidates at a time, their
-// rows staged through shared memory 32 dims at a time (coalesced; a lane
-// reading its own candidate's row would touch 32 lines a load), the distance
-// chain of knn.cu per lane, and insertion into the warp's sorted list (lane l
-// holds entry l). A query whose lists overflowed, or any query when *bad, goes
-// to left.
+// chain distances, and insertion into the warp's sorted list (lane l holds
+// entry l). A query whose lists overflowed, or any query when *bad, goes to
+// left.
 constexpr int kRefineWarps = 4;
 template <bool EUC>
 __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__restrict__ x, uint32_t n, uint32_t dim, uint32_t k,
@@ -610,9 +772,7 @@ __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__res
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t q = blockIdx.x * kRefineWarps + warp;
     if (q >= nq) return;  // warp-uniform
-    float(&S)[32][33] = sh[warp];
     const uint32_t self = qidx ? qidx[q0 + q] : q0 + q;
-    const float *xq = x + (size_t)self * dim;
     bool over = *bad != 0;
     float ld = __int_as_float(0x7f800000);
     uint32_t li = ~0u;
@@ -630,36 +790,8 @@ __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__res
                 live = false;
                 mine = self;
             }
-            const uint32_t rows = min(32u, c - b);
-            float acc = 0.0f;
-            for (uint32_t d0 = 0; d0 < dim; d0 += 32) {
-                const uint32_t w = min(32u, dim - d0);
-                __syncwarp();
-                if (w > 16) {
-#pragma unroll 8
-                    for (uint32_t r = 0; r < rows; r++) {
-                        const uint32_t id = __shfl_sync(kFull, mine, r);
-                        if (lane < w) S[r][lane] = __ldg(x + (size_t)id * dim + d0 + lane);
-                    }
-                } else {  // two rows a step
-                    for (uint32_t r = 0; r < rows; r += 2) {
-                        const uint32_t id = __shfl_sync(kFull, mine, (r + (lane >> 4)) & 31u);
-                        const uint32_t e = lane & 15;
-                        if (e < w) S[r + (lane >> 4)][e] = __ldg(x + (size_t)id * dim + d0 + e);
-                    }
-                }
-                __syncwarp();
-                for (uint32_t d = 0; d < w; d++) {
-                    const float a = __ldg(xq + d0 + d), v = S[lane][d];
-                    if (EUC) {
-                        const float df = a - v;
-                        acc = __fmaf_rn(df, df, acc);
-                    } else {
-                        acc = __fmaf_rn(a, v, acc);
-                    }
-                }
-            }
-            const float dist = EUC ? acc : 1.0f - acc;
+            const float dist =
+                chain_distance<EUC>(x, dim, x + (size_t)self * dim, mine, min(32u, c - b), sh[warp], lane);
             float td = __shfl_sync(kFull, ld, k - 1);
             uint32_t ti = __shfl_sync(kFull, li, k - 1);
             unsigned pend = __ballot_sync(kFull, live && mine != self && better(dist, mine, td, ti));
@@ -692,13 +824,200 @@ __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__res
     }
 }
 
-template <int MB, int PASS>
+// Ranks: the sorted thresholds of every query, a warp each, and their scores.
+// A point is better than a threshold T only at a chain distance of at most T,
+// so (gamma as above) surely when its true distance D is below T (1 - 2 gamma)
+// and surely not above T (1 + 2 gamma). Its score lies within kappa (u^2 +
+// v^2) of (u^2 - D) / 2 with a norm v of at most u + sqrt(D): with
+// f(D) = (u^2 - D) / 2 + kappa (u^2 + (u + sqrt D)^2), which falls in D from
+// D0 = (2 kappa u / (1 - 2 kappa))^2 on, no point at or beyond T (1 - 2 gamma)
+// scores more than hi = f(max(D0, T (1 - 2 gamma))), and none up to T (1 + 2
+// gamma) less than lo, the same with -kappa. Cosine: scores are dot products,
+// the threshold's 1 - T, the bound as in k_filter_threshold. A threshold that
+// is no number goes to *bad.
+__global__ void k_rank_bounds(const float *__restrict__ thr_d, const uint32_t *__restrict__ thr_j, uint32_t nq, uint32_t k,
+                              const float *__restrict__ norm, const uint32_t *__restrict__ qidx, uint32_t q0, uint32_t dim,
+                              bool euc, const float *__restrict__ rho, uint32_t steps, float *__restrict__ hi,
+                              float *__restrict__ lo,
+                              uint32_t *__restrict__ given, uint32_t *__restrict__ bad)
+{
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (q >= nq) return;  // warp-uniform
+    const size_t at = (size_t)(q0 + q) * k;
+    const float td = lane < k ? thr_d[at + lane] : 0.0f;
+    const uint32_t tj = lane < k ? thr_j[at + lane] : 0u;
+    if (lane < k && !(td <= FLT_MAX)) *bad = 1u;
+    uint32_t place = 0;  // a repeated neighbour keeps the order of the lanes
+    for (uint32_t m = 0; m < k; m++) {
+        const float od = __shfl_sync(kFull, td, m);
+        const uint32_t oj = __shfl_sync(kFull, tj, m);
+        place += (better(od, oj, td, tj) || (od == td && oj == tj && m < lane)) ? 1u : 0u;
+    }
+    if (lane >= k || place >= k) return;
+    const double kappa = filter_kappa(rho, steps);
+    double up, down;
+    if (euc) {
+        const double u2 = (double)norm[qidx ? qidx[q0 + q] : q0 + q], u = sqrt(u2), tiny = 1e-30;
+        const double gamma = (dim + 8) * 0x1p-24, t1 = (double)td * (1.0 - 2.0 * gamma), t2 = (double)td * (1.0 + 2.0 * gamma);
+        const double r0 = 2.0 * kappa * u / (1.0 - 2.0 * kappa), r1 = fmax(r0, sqrt(fmax(t1, 0.0))), r2 = sqrt(fmax(t2, 0.0));
+        up = 0.5 * (u2 - r1 * r1) + kappa * (u2 + (u + r1) * (u + r1)) + tiny;
+        down = 0.5 * (u2 - r2 * r2) - kappa * (u2 + (u + r2) * (u + r2)) - tiny;
+    } else {
+        const double e = 2.1 * kappa + (dim + 16.0) * 0x1p-24 + 0x1p-22;
+        up = 1.0 - (double)td + e;
+        down = 1.0 - (double)td - e;
+    }
+    const size_t o = (size_t)q * k + place;
+    hi[o] = __double2float_ru(up);
+    lo[o] = __double2float_rd(down);
+    given[o] = lane;
+}
+
+// The listed points of every query, settled by their chain distances against
+// all its thresholds (lane m holds the m-th of the sorted ones), plus the zone
+// counts: a point of zone z is better than the thresholds from z on.
+template <bool EUC>
+__global__ void __launch_bounds__(kRefineWarps * 32)
+    k_rank_refine(const float *__restrict__ x, uint32_t n, uint32_t dim, uint32_t k, const uint32_t *__restrict__ qidx,
+                  uint32_t q0, uint32_t nq, const float *__restrict__ thr_d, const uint32_t *__restrict__ thr_j,
+                  const uint32_t *__restrict__ given, const uint32_t *__restrict__ zones, const uint32_t *__restrict__ list,
+                  const uint32_t *__restrict__ count, uint32_t parts, uint32_t cap, const uint32_t *__restrict__ bad,
+                  uint32_t *__restrict__ counts, uint32_t *__restrict__ left, uint32_t *__restrict__ n_left)
+{
+    __shared__ float sh[kRefineWarps][32][33];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t q = blockIdx.x * kRefineWarps + warp;
+    if (q >= nq) return;  // warp-uniform
+    const uint32_t self = qidx ? qidx[q0 + q] : q0 + q;
+    bool over = *bad != 0;
+    const size_t at = (size_t)(q0 + q) * k;
+    uint32_t c_m = 0, g = 0, tj = 0;
+    float td = 0.0f;
+    if (!over && lane < k) {
+        c_m = zones[(size_t)q * 32 + lane];
+        g = given[(size_t)q * k + lane];
+        td = thr_d[at + g];
+        tj = thr_j[at + g];
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, c_m, off);
+        if ((int)lane >= off) c_m += u;
+    }
+    for (uint32_t p = 0; !over && p < parts; p++) {
+        const uint32_t c = count[(size_t)p * nq + q];
+        if (c > cap) {
+            over = true;
+            break;
+        }
+        const uint32_t *L = list + ((size_t)p * nq + q) * cap;
+        for (uint32_t b = 0; b < c; b += 32) {
+            const uint32_t rows = min(32u, c - b);
+            uint32_t mine = lane < rows ? L[b + lane] : self;
+            if (mine >= n) mine = self;
+            const float dist = chain_distance<EUC>(x, dim, x + (size_t)self * dim, mine, rows, sh[warp], lane);
+            for (uint32_t r = 0; r < rows; r++) {
+                const float d = __shfl_sync(kFull, dist, r);
+                const uint32_t i = __shfl_sync(kFull, mine, r);
+                c_m += (i != self && better(d, i, td, tj)) ? 1u : 0u;
+            }
+        }
+    }
+    if (over) {
+        if (lane == 0) left[atomicAdd(n_left, 1u)] = q0 + q;
+    } else if (lane < k) {
+        counts[at + g] = c_m;
+    }
+}
+
+template <int MB, int PASS, int STEPS = 0>
 void launch_filter(const FilterArgs &P, uint32_t blocks, size_t smem, cudaStream_t s)
 {
-    check_cuda(cudaFuncSetAttribute(k_filter<MB, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    check_cuda(cudaFuncSetAttribute(k_filter<MB, PASS, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "filter shared memory");
-    k_filter<MB, PASS><<<dim3(blocks, P.slices), kFilterThreads, smem, s>>>(P);
+    k_filter<MB, PASS, STEPS><<<dim3(blocks, P.slices), kFilterThreads, smem, s>>>(P);
     check_launch("k_filter");
+}
+
+// The points' operand image, norms and centre, and room for a batch's queries.
+struct Packed {
+    Pack pk;
+    DevBuf<float> mu, norm, rho;
+    DevBuf<uint4> a, b;
+    DevBuf<uint32_t> bad;
+    const float *centre = nullptr;
+    uint32_t n_tiles = 0;
+    void alloc(const KnnFilterArgs &A, uint32_t batch, cudaStream_t s)
+    {
+        pk = pack_of(A.dim);
+        n_tiles = ceil_div(A.n, kTileN);
+        mu.alloc(A.dim, s);
+        norm.alloc(A.n, s);
+        rho.alloc(2, s);
+        b.alloc((size_t)n_tiles * pk.chunks * (kBBytes / 16), s);
+        a.alloc((size_t)(batch / kBlkM) * pk.chunks * (kABytes / 16), s);
+        bad.alloc(1, s);
+    }
+    void points(const KnnFilterArgs &A, cudaStream_t s)
+    {
+        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
+        check_cuda(cudaMemsetAsync(rho.p, 0, 2 * sizeof(float), s), "memset");
+        if (A.euc) {
+            k_filter_centre<<<ceil_div(A.dim, 8), 1024, 0, s>>>(A.x, A.n, A.dim, mu.p);
+            centre = mu.p;
+        }
+        k_filter_norms<<<ceil_div((uint64_t)A.n * 32, 256), 256, 0, s>>>(A.x, A.n, A.dim, centre, pk.terms, norm.p,
+                                                                                rho.p, bad.p);
+        k_filter_pack<false><<<ceil_div((uint64_t)n_tiles * kTileN * pk.chunks * 8, 256), 256, 0, s>>>(
+            A.x, A.n, A.dim, centre, norm.p, nullptr, 0, A.n, n_tiles * kTileN, pk.terms, pk.chunks, A.euc, b.p);
+        check_launch("filter packing");
+    }
+    void queries(const KnnFilterArgs &A, uint32_t q0, uint32_t nq, uint32_t rows, cudaStream_t s)
+    {
+        k_filter_pack<true><<<ceil_div((uint64_t)rows * pk.chunks * 8, 256), 256, 0, s>>>(
+            A.x, A.n, A.dim, centre, norm.p, A.qidx, q0, nq, rows, pk.terms, pk.chunks, A.euc, a.p);
+        check_launch("filter packing");
+    }
+};
+
+// Slices of the points for `blocks` query blocks: fewest rounds of blocks over
+// the SMs, a block costing about six tiles besides its own.
+uint32_t slices_of(uint32_t blocks, uint32_t tiles)
+{
+    const uint32_t sms = (uint32_t)device_sm_count();
+    uint32_t best = 1;
+    uint64_t cost = ~0ull;
+    for (uint32_t S = 1; S <= 16 && S <= tiles; S++) {
+        const uint64_t c = (uint64_t)ceil_div((uint64_t)blocks * S, sms) * (ceil_div(tiles, S) + 6);
+        if (c < cost) {
+            cost = c;
+            best = S;
+        }
+    }
+    return best;
+}
+
+// The most (blocks x slices) of any batch.
+uint32_t most_items(uint32_t nq, uint32_t batch, uint32_t rows, uint32_t tiles)
+{
+    uint32_t most = 1;
+    for (uint32_t q0 = 0; q0 < nq; q0 += batch) {
+        const uint32_t blocks = ceil_div(std::min(batch, nq - q0), rows);
+        most = std::max(most, slices_of(blocks, tiles) * blocks);
+    }
+    return most;
+}
+
+// Shared memory of k_filter<1, 3> behind A and the ring: hi, lo, zone counters.
+uint32_t rank_steps(uint32_t k) { return k < 16 ? 4 : 5; }
+size_t rank_smem(uint32_t k)
+{
+    return sizeof(float) * kBlkM * (((size_t)1 << rank_steps(k)) - 1 + k + 1) + sizeof(uint32_t) * 512 * (k + 1);
+}
+uint32_t rank_stages(uint32_t chunks, uint32_t k)
+{
+    const size_t fixed = 2048 + (size_t)chunks * kABytes + rank_smem(k);
+    return fixed >= kSmemMax ? 0u : (uint32_t)std::min<size_t>(5, (kSmemMax - fixed) / kBBytes);
 }
 
 }  // namespace
@@ -727,79 +1046,47 @@ bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaSt
     // points of all reach it
     const double r = -(double)kGroups * std::log(1.0 - (double)(A.k + 1) / kGroups);
     const uint32_t stride = std::max(1u, std::min((uint32_t)(kHitTarget / r), n_tiles / 4));
-    // queries in batches of at most two waves of blocks: bounds the scratch
-    const uint32_t rows = MB * kBlkM, batch = std::min<uint32_t>(ceil_div(A.nq, rows), 2 * MB == 4 ? 2 * sms : 4 * sms) * rows;
-    // slices of the points: fewest rounds of blocks over the SMs, a block
-    // costing about six tiles besides its own
-    auto slices_of = [&](uint32_t blocks, uint32_t tiles) {
-        uint32_t best = 1;
-        uint64_t cost = ~0ull;
-        for (uint32_t S = 1; S <= 16 && S <= tiles; S++) {
-            const uint64_t c = (uint64_t)ceil_div((uint64_t)blocks * S, sms) * (ceil_div(tiles, S) + 6);
-            if (c < cost) {
-                cost = c;
-                best = S;
-            }
-        }
-        return best;
-    };
+    // queries in batches of at most two waves of blocks (four with one block of
+    // queries each): bounds the scratch
+    const uint32_t rows = MB * kBlkM, batch = std::min<uint32_t>(ceil_div(A.nq, rows), (MB == 2 ? 2 : 4) * sms) * rows;
     const uint32_t sampled = ceil_div(n_tiles, stride);
-    uint32_t most1 = 1, most2 = 1;
-    for (uint32_t q0 = 0; q0 < A.nq; q0 += batch) {
-        const uint32_t blocks = ceil_div(std::min(batch, A.nq - q0), rows);
-        most1 = std::max(most1, slices_of(blocks, sampled) * blocks);
-        most2 = std::max(most2, slices_of(blocks, n_tiles) * blocks);
-    }
+    const uint32_t most1 = most_items(A.nq, batch, rows, sampled), most2 = most_items(A.nq, batch, rows, n_tiles);
     const uint32_t per = MB == 2 ? 1 : 2;  // accumulators of a slice
-    DevBuf<float> mu, norm, gmax, least;
-    DevBuf<uint4> pa, pb;
-    DevBuf<uint32_t> list, count, bad;
+    Packed K;
+    DevBuf<float> gmax, least;
+    DevBuf<uint32_t> list, count;
     try {
-        mu.alloc(A.dim, s);
-        norm.alloc(A.n, s);
-        pb.alloc((size_t)n_tiles * C * (kBBytes / 16), s);
-        pa.alloc((size_t)(batch / kBlkM) * C * (kABytes / 16), s);
+        K.alloc(A, batch, s);
         gmax.alloc((size_t)most1 * per * rows * kGroups, s);
         least.alloc(batch, s);
         // a part's list (a slice's, of one half of the columns) holds its
         // share of kListCap and 64 more
         list.alloc((size_t)most2 * per * 2 * rows * 64 + (size_t)batch * kListCap, s);
         count.alloc((size_t)most2 * per * 2 * rows, s);
-        bad.alloc(1, s);
     } catch (const Error &e) {
         if (e.status != UMAPCU_CUDA_ALLOC) throw;
         return false;
     }
-    check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
-    const float *centre = nullptr;
-    if (A.euc) {
-        k_filter_centre<<<ceil_div(A.dim, 8), 1024, 0, s>>>(A.x, A.n, A.dim, mu.p);
-        centre = mu.p;
-    }
-    k_filter_norms<<<ceil_div((uint64_t)A.n * 32, 256), 256, 0, s>>>(A.x, A.n, A.dim, centre, norm.p, bad.p);
-    k_filter_pack<false><<<ceil_div((uint64_t)n_tiles * kTileN * C * 8, 256), 256, 0, s>>>(
-        A.x, A.n, A.dim, centre, norm.p, nullptr, 0, A.n, n_tiles * kTileN, pk.terms, C, A.euc, pb.p);
-    check_launch("filter packing");
+    K.points(A, s);
     for (uint32_t q0 = 0; q0 < A.nq; q0 += batch) {
         const uint32_t nq = std::min(batch, A.nq - q0), blocks = ceil_div(nq, rows);
-        k_filter_pack<true><<<ceil_div((uint64_t)blocks * rows * C * 8, 256), 256, 0, s>>>(
-            A.x, A.n, A.dim, centre, norm.p, A.qidx, q0, nq, blocks * rows, pk.terms, C, A.euc, pa.p);
+        K.queries(A, q0, nq, blocks * rows, s);
         FilterArgs P{};
-        P.a = pa.p;
-        P.b = pb.p;
+        P.a = K.a.p;
+        P.b = K.b.p;
         P.nq = nq;
         P.n_tiles = n_tiles;
         P.chunks = C;
         P.steps = pk.steps;
         P.stages = stages;
-        P.bad = bad.p;
+        P.bad = K.bad.p;
         P.stride = stride;
         P.slices = slices_of(blocks, sampled);
         P.gmax = gmax.p;
         if (MB == 2) launch_filter<2, 1>(P, blocks, smem, s);
         else launch_filter<1, 1>(P, blocks, smem, s);
         k_filter_threshold<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(
-            gmax.p, P.slices * per, nq, A.k, norm.p, A.qidx, q0, A.dim, A.euc, filter_kappa(pk.terms), least.p);
+            gmax.p, P.slices * per, nq, A.k, K.norm.p, A.qidx, q0, A.dim, A.euc, K.rho.p, pk.steps, least.p);
         check_launch("k_filter_threshold");
         P.stride = 1;
         P.slices = slices_of(blocks, n_tiles);
@@ -813,11 +1100,89 @@ bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaSt
         const unsigned rg = ceil_div(nq, kRefineWarps);
         if (A.euc)
             k_refine<true><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, list.p, count.p, parts,
-                                                            P.cap, bad.p, A.out_idx, A.out_dist, left, n_left);
+                                                            P.cap, K.bad.p, A.out_idx, A.out_dist, left, n_left);
         else
             k_refine<false><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, list.p, count.p, parts,
-                                                             P.cap, bad.p, A.out_idx, A.out_dist, left, n_left);
+                                                             P.cap, K.bad.p, A.out_idx, A.out_dist, left, n_left);
         check_launch("k_refine");
+    }
+    return true;
+}
+
+bool rank_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k)
+{
+    return knn_filter_takes(n, dim, nq, k) && k < 32 && rank_stages(pack_of(dim).chunks, k) >= 2;
+}
+
+bool rank_filter(const KnnFilterArgs &A, const float *thr_d, const uint32_t *thr_j, uint32_t *counts, uint32_t *left,
+                 uint32_t *n_left, cudaStream_t s)
+{
+    const Pack pk = pack_of(A.dim);
+    const uint32_t C = pk.chunks, n_tiles = ceil_div(A.n, kTileN), stages = rank_stages(C, A.k);
+    const size_t smem = (size_t)C * kABytes + (size_t)stages * kBBytes + rank_smem(A.k) + 1024;
+    // at most 16 384 queries at a time: a query's lists hold 4096 points and 64
+    // more a part
+    constexpr uint32_t kRankCap = 4096;
+    const uint32_t batch = std::min<uint32_t>(ceil_div(A.nq, kBlkM), 128) * kBlkM;
+    const uint32_t most = most_items(A.nq, batch, kBlkM, n_tiles);
+    Packed K;
+    DevBuf<float> hi, lo;
+    DevBuf<uint32_t> given, zones, list, count;
+    try {
+        K.alloc(A, batch, s);
+        hi.alloc((size_t)batch * A.k, s);
+        lo.alloc((size_t)batch * A.k, s);
+        given.alloc((size_t)batch * A.k, s);
+        zones.alloc((size_t)batch * 32, s);
+        list.alloc((size_t)most * 4 * kBlkM * 64 + (size_t)batch * kRankCap, s);
+        count.alloc((size_t)most * 4 * kBlkM, s);
+    } catch (const Error &e) {
+        if (e.status != UMAPCU_CUDA_ALLOC) throw;
+        return false;
+    }
+    K.points(A, s);
+    for (uint32_t q0 = 0; q0 < A.nq; q0 += batch) {
+        const uint32_t nq = std::min(batch, A.nq - q0), blocks = ceil_div(nq, kBlkM);
+        K.queries(A, q0, nq, blocks * kBlkM, s);
+        k_rank_bounds<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(thr_d, thr_j, nq, A.k, K.norm.p, A.qidx, q0, A.dim,
+                                                                       A.euc, K.rho.p, pk.steps, hi.p, lo.p, given.p,
+                                                                       K.bad.p);
+        check_launch("k_rank_bounds");
+        check_cuda(cudaMemsetAsync(zones.p, 0, sizeof(uint32_t) * 32 * nq, s), "memset");
+        FilterArgs P{};
+        P.a = K.a.p;
+        P.b = K.b.p;
+        P.nq = nq;
+        P.n_tiles = n_tiles;
+        P.chunks = C;
+        P.steps = pk.steps;
+        P.stages = stages;
+        P.bad = K.bad.p;
+        P.stride = 1;
+        P.slices = slices_of(blocks, n_tiles);
+        P.list = list.p;
+        P.count = count.p;
+        P.k = A.k;
+        P.zone_rows = (1u << rank_steps(A.k)) - 1;
+        P.hi = hi.p;
+        P.lo = lo.p;
+        P.qidx = A.qidx;
+        P.q0 = q0;
+        P.zones = zones.p;
+        const uint32_t parts = P.slices * 4;
+        P.cap = kRankCap / parts + 64;
+        if (rank_steps(A.k) == 4) launch_filter<1, 3, 4>(P, blocks, smem, s);
+        else launch_filter<1, 3, 5>(P, blocks, smem, s);
+        const unsigned rg = ceil_div(nq, kRefineWarps);
+        if (A.euc)
+            k_rank_refine<true><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, thr_d, thr_j, given.p,
+                                                                 zones.p, list.p, count.p, parts, P.cap, K.bad.p, counts,
+                                                                 left, n_left);
+        else
+            k_rank_refine<false><<<rg, kRefineWarps * 32, 0, s>>>(A.x, A.n, A.dim, A.k, A.qidx, q0, nq, thr_d, thr_j, given.p,
+                                                                  zones.p, list.p, count.p, parts, P.cap, K.bad.p, counts,
+                                                                  left, n_left);
+        check_launch("k_rank_refine");
     }
     return true;
 }

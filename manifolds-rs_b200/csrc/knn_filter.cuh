@@ -27,4 +27,12 @@ bool knn_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k);
 // device memory for its scratch, nothing was done.
 bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaStream_t s);
 
+// The same for ranks: counts [nq][k] = points strictly before each threshold
+// (thr_d, thr_j) [nq][k] of the query by (distance, index), itself excluded
+// (A.out_idx and A.out_dist are not used). Counts of queries in left are not
+// written.
+bool rank_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k);
+bool rank_filter(const KnnFilterArgs &A, const float *thr_d, const uint32_t *thr_j, uint32_t *counts, uint32_t *left,
+                 uint32_t *n_left, cudaStream_t s);
+
 }  // namespace umapcu

@@ -81,3 +81,29 @@ def test_filter_query_subset():
     q = umapcu.embedding_quality(X, Y, ki.astype(np.int32), 15, queries=sub)
     assert q["trust"] == O.trustworthiness(X, Y, 15, queries=sub)
     assert q["knn_preservation"] == pytest.approx(O.knn_preservation(ki, Y, 15, queries=sub), abs=1e-12)
+
+
+# 15 / 16 neighbours: four and five steps of the search; 31: the most, 32: the
+# tile kernel; dims 63 / 64: chunks; 191: too wide beside the rank tables; Y
+# unrelated to X: thresholds all over the distances
+@pytest.mark.parametrize("n,dim,k,metric,kind", [(2048, 3, 15, "euclidean", "plain"), (3001, 50, 16, "euclidean", "plain"),
+                                                 (2500, 63, 31, "euclidean", "plain"), (2500, 64, 32, "euclidean", "plain"),
+                                                 (2600, 100, 15, "cosine", "plain"), (2100, 191, 15, "euclidean", "plain"),
+                                                 (3000, 10, 15, "euclidean", "ties"), (3000, 8, 1, "cosine", "ties"),
+                                                 (4000, 12, 15, "euclidean", "offset"), (3000, 12, 15, "euclidean", "duplicates"),
+                                                 (2500, 6, 15, "euclidean", "infinite")])
+def test_rank_filter_counts(n, dim, k, metric, kind):
+    rng = np.random.default_rng(n + dim + k)
+    X = rng.normal(size=(n, dim)).astype(np.float32)
+    if kind == "ties":
+        X = np.round(X).astype(np.float32) + 1.0
+    elif kind == "offset":  # every point within the bound of every threshold: lists overflow
+        X = (X * 1e-3 + 1000.0 * np.sign(X[:, :1])).astype(np.float32)
+    elif kind == "duplicates":
+        X[: n // 2] = X[0]
+    elif kind == "infinite":
+        X[5, 1] = 1e20
+    Y = rng.normal(size=(n, 2)).astype(np.float32)
+    q = rng.choice(n, 700, replace=False).astype(np.uint32)
+    got = umapcu.embedding_quality(X, Y, None, k, queries=q, dist_metric=metric)
+    assert got["trust"] == O.trustworthiness(X, Y, k, queries=q, metric=umapcu._metric(metric))
