@@ -536,8 +536,6 @@ umapcu_status umapcu_construct_umap_graph(const int32_t *knn_idx, const float *k
         const uint64_t nk = (uint64_t)n * k;
         if (capacity < 2 * nk) return UMAPCU_CAPACITY;
         if (!row || !col || !val) return UMAPCU_BAD_ARG;
-        for (uint64_t i = 0; i < nk; i++)
-            if (knn_idx[i] < 0 || (uint32_t)knn_idx[i] >= n) return UMAPCU_BAD_ARG;
         NvtxRange r("umapcu construct_umap_graph");
         Stream S;
         DevBuf<int32_t> di(nk, S.s);
@@ -565,20 +563,26 @@ umapcu_status umapcu_dens_state_new(uint32_t n, uint64_t nnz, const uint32_t *ro
         if (n == 0) return UMAPCU_NO_DATA;
         if (!r || !mu_sum || !mu_tot || !knn_idx || !knn_dist || k == 0) return UMAPCU_BAD_ARG;
         if (nnz && (!row || !col || !val)) return UMAPCU_BAD_ARG;
-        for (uint64_t e = 0; e < nnz; e++)
-            if (row[e] >= n || col[e] >= n || (e && row[e] < row[e - 1])) return UMAPCU_BAD_ARG;
         const uint64_t nk = (uint64_t)n * k;
-        for (uint64_t i = 0; i < nk; i++)
-            if (knn_idx[i] < 0 || (uint32_t)knn_idx[i] >= n) return UMAPCU_BAD_ARG;
         Stream S;
-        DevBuf<uint32_t> dr(nnz, S.s), dc(nnz, S.s);
+        DevBuf<uint32_t> dr(nnz, S.s), dc(nnz, S.s), bad(1, S.s);
         DevBuf<float> dv(nnz, S.s), dd(nk, S.s), outr(n, S.s), outm(n, S.s);
         DevBuf<int32_t> di(nk, S.s);
         h2d(dr.p, row, nnz, S.s);
         h2d(dc.p, col, nnz, S.s);
-        h2d(dv.p, val, nnz, S.s);
         h2d(di.p, knn_idx, nk, S.s);
+        // the indices are checked before anything reads at their places (a
+        // negative neighbour is one past any n)
+        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), S.s), "memset");
+        check_range_dev(dr.p, nnz, n, true, bad.p, S.s);
+        check_range_dev(dc.p, nnz, n, false, bad.p, S.s);
+        check_range_dev((const uint32_t *)di.p, nk, std::min(n, 1u << 31), false, bad.p, S.s);
+        h2d(dv.p, val, nnz, S.s);
         h2d(dd.p, knn_dist, nk, S.s);
+        uint32_t bad_h = 0;
+        d2h(&bad_h, bad.p, 1, S.s);
+        sync(S.s);
+        if (bad_h) return UMAPCU_BAD_ARG;
         umapcu_status rc =
             dens_state_dev(n, nnz, dr.p, dc.p, dv.p, di.p, dd.p, k, distances_squared, outr.p, outm.p, mu_tot, S.s);
         if (rc != UMAPCU_OK) return rc;

@@ -92,11 +92,35 @@ void smooth_knn_dist_dev(const float *d_dist, uint32_t n, uint32_t k, float loca
     check_launch("k_smooth_knn_dist");
 }
 
+// Index checks of the callers' arrays, on the device: reading them once more
+// on the host took longer than the kernels behind it (15M neighbours 8 ms, a
+// 6M-entry graph 6 ms). *bad is set when an index is outside [0, limit), or,
+// ASCENDING, below the one before it.
+template <bool ASCENDING>
+__global__ void k_check_range(const uint32_t *__restrict__ v, uint64_t m, uint32_t limit, uint32_t *__restrict__ bad)
+{
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    bool wrong = false;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += step)
+        wrong = wrong || v[i] >= limit || (ASCENDING && i && v[i] < v[i - 1]);
+    if (wrong) *bad = 1u;
+}
+
+void check_range_dev(const uint32_t *d_v, uint64_t m, uint32_t limit, bool ascending, uint32_t *d_bad, cudaStream_t s)
+{
+    if (!m) return;
+    const unsigned grid = (unsigned)std::min<uint64_t>((m + 255) / 256, 8ull * (unsigned)device_sm_count());
+    if (ascending) k_check_range<true><<<grid, 256, 0, s>>>(d_v, m, limit, d_bad);
+    else k_check_range<false><<<grid, 256, 0, s>>>(d_v, m, limit, d_bad);
+    check_launch("k_check_range");
+}
+
 // graph.rs:625-653: membership weight of every kNN entry; keep[] marks
-// non-self entries.
+// non-self entries. *bad is set by a neighbour outside [0, n) (nothing here or
+// behind it reads at a neighbour's place).
 __global__ void k_knn_weights(const int32_t *__restrict__ idx, const float *__restrict__ dist, uint32_t n,
                               uint32_t k, const float *__restrict__ sigma, const float *__restrict__ rho,
-                              float *__restrict__ w_out, uint32_t *__restrict__ keep)
+                              float *__restrict__ w_out, uint32_t *__restrict__ keep, uint32_t *__restrict__ bad)
 {
     uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (uint64_t)n * k) return;
@@ -110,7 +134,9 @@ __global__ void k_knn_weights(const int32_t *__restrict__ idx, const float *__re
     else if (adjusted > 0.0f) w = 0.0f;
     else w = 1.0f;
     w_out[p] = w;
-    keep[p] = (uint32_t)idx[p] != i;
+    const uint32_t j = (uint32_t)idx[p];
+    if (j >= n) *bad = 1u;
+    keep[p] = j != i;
 }
 
 __global__ void k_compact_coo(const int32_t *__restrict__ idx, const float *__restrict__ w, uint64_t m,
@@ -247,10 +273,13 @@ void construct_graph_dev(const int32_t *d_idx, const float *d_dist, uint32_t n, 
 
     // knn_to_coo
     DevBuf<float> w(nk, s);
-    DevBuf<uint32_t> keep(nk, s), pos(nk, s);
-    k_knn_weights<<<ceil_div(nk, 256), 256, 0, s>>>(d_idx, d_dist, n, k, d_sigma, d_rho, w.p, keep.p);
+    DevBuf<uint32_t> keep(nk, s), pos(nk, s), bad(1, s);
+    check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
+    k_knn_weights<<<ceil_div(nk, 256), 256, 0, s>>>(d_idx, d_dist, n, k, d_sigma, d_rho, w.p, keep.p, bad.p);
     check_launch("k_knn_weights");
-    uint64_t m = scan_flags(keep.p, pos.p, nk, s);
+    uint32_t bad_h = 0;
+    uint64_t m = scan_flags(keep.p, pos.p, nk, s, bad.p, &bad_h);
+    if (bad_h) fail(UMAPCU_BAD_ARG, "kNN index out of range");
     DevBuf<uint32_t> row(m, s), col(m, s);
     DevBuf<float> val(m, s);
     if (m) {
@@ -786,26 +815,48 @@ __global__ void k_orig_radii(const uint32_t *__restrict__ row, const float *__re
     ro[i] = log(1e-8 + a / denom);
 }
 
-// Deterministic single-block f64 reductions (fixed thread count and order).
+// Deterministic f64 sums (fixed thread counts and order): kSumBlocks blocks sum
+// a grid-strided share each, the last to finish (ticket) adds their sums in
+// order. One block alone took 93 us at 200k points. MODE 0: the mean of x, 1:
+// the sum of squared differences from *mean_in, 2: the sum of xf.
+constexpr unsigned kSumBlocks = 128;
 template <int MODE>
-__global__ void k_block_sum(const double *__restrict__ x, const float *__restrict__ xf, uint64_t n,
-                            const double *__restrict__ mean_in, double *__restrict__ out)
+__global__ void __launch_bounds__(256) k_sum(const double *__restrict__ x, const float *__restrict__ xf, uint64_t n,
+                                             const double *__restrict__ mean_in, double *__restrict__ part,
+                                             uint32_t *__restrict__ ticket, double *__restrict__ out)
 {
-    __shared__ double sh[1024];
+    __shared__ double sh[256];
+    __shared__ bool last;
+    const double mean = MODE == 1 ? *mean_in : 0.0;
+    auto block_sum = [&](double acc) {
+        sh[threadIdx.x] = acc;
+        __syncthreads();
+        for (int w = 128; w > 0; w >>= 1) {
+            if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+            __syncthreads();
+        }
+        return sh[0];
+    };
     double acc = 0.0;
-    double mean = MODE == 1 ? *mean_in : 0.0;
-    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    for (uint64_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += kSumBlocks * 256u) {
         if (MODE == 0) acc += x[i];
         else if (MODE == 1) { double d = x[i] - mean; acc += d * d; }
         else acc += (double)xf[i];
     }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
+    const double mine = block_sum(acc);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = mine;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == kSumBlocks - 1;
     }
-    if (threadIdx.x == 0) out[0] = MODE == 0 ? sh[0] / (double)n : (MODE == 1 ? sh[0] : sh[0]);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const double all = block_sum(threadIdx.x < kSumBlocks ? __ldcg(part + threadIdx.x) : 0.0);
+    if (threadIdx.x == 0) {
+        out[0] = MODE == 0 ? all / (double)n : all;
+        *ticket = 0u;
+    }
 }
 
 __global__ void k_standardise(const double *__restrict__ ro, const double *__restrict__ ms, uint32_t n,
@@ -830,12 +881,14 @@ umapcu_status dens_state_dev(uint32_t n, uint64_t nnz, const uint32_t *d_row, co
         k_edge_dsq<<<ceil_div(nnz, 256), 256, 0, s>>>(d_row, d_col, nnz, d_idx, d_dist, k, distances_squared, dsq.p);
         check_launch("k_edge_dsq");
     }
-    DevBuf<double> ro(n, s), ms(n, s), scal(3, s);
+    DevBuf<double> ro(n, s), ms(n, s), scal(3, s), part(kSumBlocks, s);
+    DevBuf<uint32_t> ticket(1, s);
+    check_cuda(cudaMemsetAsync(ticket.p, 0, sizeof(uint32_t), s), "memset");
     k_orig_radii<<<ceil_div(n, 256), 256, 0, s>>>(d_row, d_val, dsq.p, nnz, n, ro.p, ms.p);
     check_launch("k_orig_radii");
-    k_block_sum<0><<<1, 1024, 0, s>>>(ro.p, nullptr, n, nullptr, scal.p);
-    k_block_sum<1><<<1, 1024, 0, s>>>(ro.p, nullptr, n, scal.p, scal.p + 1);
-    check_launch("k_block_sum");
+    k_sum<0><<<kSumBlocks, 256, 0, s>>>(ro.p, nullptr, n, nullptr, part.p, ticket.p, scal.p);
+    k_sum<1><<<kSumBlocks, 256, 0, s>>>(ro.p, nullptr, n, scal.p, part.p, ticket.p, scal.p + 1);
+    check_launch("k_sum");
     double h[2];
     d2h(h, scal.p, 2, s);
     sync(s);
@@ -843,8 +896,8 @@ umapcu_status dens_state_dev(uint32_t n, uint64_t nnz, const uint32_t *d_row, co
     if (std::isnan(sd) || sd <= DBL_EPSILON) return UMAPCU_DEGENERATE_LOCAL_RADII;
     k_standardise<<<ceil_div(n, 256), 256, 0, s>>>(ro.p, ms.p, n, scal.p, scal.p + 1, d_r, d_mu_sum);
     check_launch("k_standardise");
-    k_block_sum<2><<<1, 1024, 0, s>>>(nullptr, d_mu_sum, n, nullptr, scal.p + 2);
-    check_launch("k_block_sum");
+    k_sum<2><<<kSumBlocks, 256, 0, s>>>(nullptr, d_mu_sum, n, nullptr, part.p, ticket.p, scal.p + 2);
+    check_launch("k_sum");
     double t = 0.0;
     d2h(&t, scal.p + 2, 1, s);
     sync(s);

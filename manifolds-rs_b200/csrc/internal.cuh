@@ -174,10 +174,15 @@ void smooth_knn_dist_dev(const float *d_dist, uint32_t n, uint32_t k, float loca
                          float bandwidth, uint32_t n_iter, float *d_sigma, float *d_rho, cudaStream_t s);
 
 // The full graph stage (lib.rs:296-306) on device buffers; the kNN arrays
-// stay owned by the caller.
+// stay owned by the caller. Fails with UMAPCU_BAD_ARG on a neighbour outside
+// [0, n).
 void construct_graph_dev(const int32_t *d_idx, const float *d_dist, uint32_t n, uint32_t k,
                          const umapcu_graph_params &gp, uint32_t n_epochs, DeviceCoo &out,
                          float *d_sigma, float *d_rho, cudaStream_t s);
+
+// Sets *d_bad when one of m indices is outside [0, limit) or, if ascending, below
+// the one before it (graph.cu).
+void check_range_dev(const uint32_t *d_v, uint64_t m, uint32_t limit, bool ascending, uint32_t *d_bad, cudaStream_t s);
 
 // densMAP constant state (density.rs:181-201) on device buffers.
 umapcu_status dens_state_dev(uint32_t n, uint64_t nnz, const uint32_t *d_row, const uint32_t *d_col,

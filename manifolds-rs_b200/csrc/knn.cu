@@ -694,10 +694,10 @@ umapcu_status umapcu_fuzzy_cross_entropy(const uint32_t *row, const uint32_t *co
     return guard_k([&]() -> umapcu_status {
         if (n == 0) return UMAPCU_NO_DATA;
         if (!y || !out || n_dim == 0 || (nnz && (!row || !col || !w))) return UMAPCU_BAD_ARG;
-        for (uint64_t e = 0; e < nnz; e++)
-            if (row[e] >= n || col[e] >= n) return UMAPCU_BAD_ARG;
-        *out = 0.0;
-        if (!nnz) return UMAPCU_OK;
+        if (!nnz) {
+            *out = 0.0;
+            return UMAPCU_OK;
+        }
         keep_pool_memory();
         Stream st;
         cudaStream_t s = st.s;
@@ -705,8 +705,17 @@ umapcu_status umapcu_fuzzy_cross_entropy(const uint32_t *row, const uint32_t *co
         DevBuf<float> dw(nnz, s), dy((size_t)n * n_dim, s);
         h2d(dr.p, row, nnz, s);
         h2d(dc.p, col, nnz, s);
+        DevBuf<uint32_t> bad(1, s);
+        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
+        check_range_dev(dr.p, nnz, n, false, bad.p, s);
+        check_range_dev(dc.p, nnz, n, false, bad.p, s);
         h2d(dw.p, w, nnz, s);
         h2d(dy.p, y, (size_t)n * n_dim, s);
+        uint32_t bad_h = 0;
+        d2h(&bad_h, bad.p, 1, s);
+        sync(s);
+        if (bad_h) return UMAPCU_BAD_ARG;
+        *out = 0.0;
         const unsigned blocks = ceil_div(nnz, 256);
         DevBuf<double> part(blocks, s);
         k_fuzzy_ce<<<blocks, 256, 0, s>>>(dr.p, dc.p, dw.p, nnz, dy.p, n_dim, (double)a, (double)b, part.p);
