@@ -129,10 +129,18 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_persistent(const Batch
     }
 }
 
+// One launch per epoch, each overlapping the one before as the single-problem
+// kernels do (grid_wait in load_segment). The fast two-dimensional form runs at
+// ten blocks an SM with half-word pieces, like theirs: 48 problems of 0.5-20k
+// points, 100 epochs, whole run @BATCH.
+template <int D, int NR, bool FAST, bool BITS>
+constexpr bool batch_dense() { return FAST && BITS && D == 2 && NR == 5; }
 template <int D, int NR, int KU, bool FAST = false, bool BITS = false>
-__global__ void __launch_bounds__(kWarps * 32, 8) k_batch_epoch(const BatchArgs B, uint32_t e)
+__global__ void __launch_bounds__(kWarps * 32, batch_dense<D, NR, FAST, BITS>() ? 10 : 8)
+    k_batch_epoch(const BatchArgs B, uint32_t e)
 {
-    __shared__ WarpSmem<D, KU, BITS, false> smem[kWarps];
+    constexpr int BP = batch_dense<D, NR, FAST, BITS>() ? 16 : 32;
+    __shared__ WarpSmem<D, KU, BITS, false, BP> smem[kWarps];
     __shared__ EpochArgs sargs[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t s = blockIdx.x * kWarps + warp;
@@ -146,7 +154,23 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_epoch(const BatchArgs 
         sargs[warp] = A;
     }
     __syncwarp();
-    epoch_segment<D, false, NR, false, KU, FAST, false, BITS>(sargs[warp], smem[warp], (s - P.seg_base) * 32u, lane);
+    epoch_segment<D, false, NR, true, KU, FAST, false, BITS, BP>(sargs[warp], smem[warp], (s - P.seg_base) * 32u, lane);
+}
+
+// k_batch_epoch behind the stream's last kernel, whose end it waits for itself.
+inline void launch_batch_epoch(void (*kernel)(BatchArgs, uint32_t), unsigned grid, const BatchArgs &B, uint32_t e,
+                               cudaStream_t s)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    check_cuda(cudaLaunchKernelEx(&cfg, kernel, B, e), "k_batch_epoch");
 }
 
 struct BatchConfig {
@@ -167,8 +191,8 @@ inline void launch_batch_kernel_t(const BatchArgs &B, const BatchConfig &c, cuda
         else k_batch_persistent<D, 5, 8, FAST, BITS><<<grid, kWarps * 32, 0, s>>>(B);
     } else {
         const unsigned grid = ceil_div(B.n_segs, kWarps);
-        if (c.ku == 4) k_batch_epoch<D, 5, 4, FAST, BITS><<<grid, kWarps * 32, 0, s>>>(B, epoch);
-        else k_batch_epoch<D, 5, 8, FAST, BITS><<<grid, kWarps * 32, 0, s>>>(B, epoch);
+        if (c.ku == 4) launch_batch_epoch(k_batch_epoch<D, 5, 4, FAST, BITS>, grid, B, epoch, s);
+        else launch_batch_epoch(k_batch_epoch<D, 5, 8, FAST, BITS>, grid, B, epoch, s);
     }
     check_launch("k_batch");
 }
@@ -199,9 +223,9 @@ inline void launch_batch_kernel_nr0(const BatchArgs &B, const BatchConfig &c, cu
         else k_batch_persistent<D, 0, 8><<<grid, kWarps * 32, 0, s>>>(B);
     } else {
         const unsigned grid = ceil_div(B.n_segs, kWarps);
-        if (bits) k_batch_epoch<D, 0, 8, false, true><<<grid, kWarps * 32, 0, s>>>(B, epoch);
-        else if (c.ku == 4) k_batch_epoch<D, 0, 4><<<grid, kWarps * 32, 0, s>>>(B, epoch);
-        else k_batch_epoch<D, 0, 8><<<grid, kWarps * 32, 0, s>>>(B, epoch);
+        if (bits) launch_batch_epoch(k_batch_epoch<D, 0, 8, false, true>, grid, B, epoch, s);
+        else if (c.ku == 4) launch_batch_epoch(k_batch_epoch<D, 0, 4>, grid, B, epoch, s);
+        else launch_batch_epoch(k_batch_epoch<D, 0, 8>, grid, B, epoch, s);
     }
     check_launch("k_batch");
 }

@@ -83,6 +83,19 @@ __device__ __forceinline__ bool checked_ok(bool ok, uint32_t *err)
 #endif
 }
 
+// Programmatic dependent launch. An epoch's kernel waits for the previous one
+// before it touches what that one writes (grid_wait) and then lets the next
+// one's blocks start as soon as all its own have come this far (grid_trigger):
+// launch latency, the tail of a kernel's last blocks and the loads of a
+// segment's row starts overlap. (Triggered before the wait, the blocks of
+// several epochs pile up and the last of them are packed onto the few SMs with
+// room: 14 -> 24 us an epoch at 50k points.) Both are no-ops in a kernel launched
+// without the attribute (launch_after). What the previous kernel writes is
+// written while this one may already run, so it is never read through the
+// non-coherent path or kept in L1 (COH below).
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // L2 residency: the embedding (gathered at random every epoch) is loaded
 // with an evict_last policy; the CSR arrays (streamed once per epoch) with
 // the streaming (evict-first) qualifier, so they do not push the embedding
@@ -97,8 +110,9 @@ __device__ __forceinline__ uint64_t l2_keep_policy()
 }
 
 // COH = true: loads of data that other SMs rewrite while the kernel runs
-// (the persistent multi-problem kernel: the embedding buffers, moments and
-// cursors change roles every epoch). They go through L2 (ld.global.cg)
+// (the epoch kernels, which overlap the previous epoch's, and the persistent
+// multi-problem kernel: the embedding buffers, moments and cursors change
+// roles every epoch). They go through L2 (ld.global.cg)
 // instead of the non-coherent read-only path / L1.
 template <int D, bool COH = false>
 __device__ __forceinline__ void load_row_keep(const float *__restrict__ y, uint32_t i, float (&out)[D], uint64_t pol)
@@ -234,6 +248,7 @@ struct WarpSmem {
     float ys[32][D];
     float part[32][D];
     float4 dn[DENS ? 32 : 1];
+    float st[DENS ? 5 : 1];  // dens_stats
 };
 
 __device__ __forceinline__ uint32_t local_node(const uint32_t *beg, uint32_t p)
@@ -329,7 +344,7 @@ __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, b
         float4 dno;
         float mu_e = 1.0f;
         if constexpr (DENS) {
-            dno = __ldg(A.dens_node + o);
+            dno = COH ? __ldcg(A.dens_node + o) : __ldg(A.dens_node + o);
             mu_e = __ldg(A.mu_entry + p);
         }
         // attractive (umap_optimiser_gpu.rs:746-762)
@@ -455,6 +470,8 @@ __device__ __forceinline__ void load_segment(const EpochArgs &A, Smem &S, uint32
     const bool valid = node < A.n;
     S.beg[lane] = A.offsets[valid ? node : A.n];
     if (lane == 31) S.beg[32] = A.offsets[min(node0 + 32u, A.n)];
+    grid_wait();  // the positions, moments and cursors are the previous epoch's
+    grid_trigger();
     if (valid) load_row<D, COH>(A.y_cur, node, ys);
     else {
 #pragma unroll
@@ -463,7 +480,8 @@ __device__ __forceinline__ void load_segment(const EpochArgs &A, Smem &S, uint32
 #pragma unroll
     for (int d = 0; d < D; d++) S.ys[lane][d] = ys[d];
     if constexpr (DENS) {
-        if (valid) S.dn[lane] = __ldg(A.dens_node + node);
+        if (valid) S.dn[lane] = COH ? __ldcg(A.dens_node + node) : __ldg(A.dens_node + node);
+        if (lane < 5) S.st[lane] = __ldcg(A.dens_stats + lane);
     }
 #ifdef UMAPCU_CHECKED
     // the segment's row starts must be in order and within the entries; a
@@ -525,7 +543,7 @@ __device__ __forceinline__ void epoch_segment(const EpochArgs &A, WarpSmem<D, KU
     const bool valid = node < A.n;
     float ys[D];
     load_segment<D, DENS, COH>(A, S, node0, lane, ys);
-    const float *dstat = A.dens_stats;
+    const float *dstat = S.st;
     // Degenerate self beyond the last beg (beg[32] read by the search only
     // through j + step <= 31 + 1).
     float g[D];
@@ -697,9 +715,9 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
     const uint32_t node = node0 + lane;
     const bool valid = node < A.n;
     float ys[D];
-    if (warp == 0) load_segment<D, DENS, false>(A, S, node0, lane, ys);
+    if (warp == 0) load_segment<D, DENS, true>(A, S, node0, lane, ys);
     __syncthreads();
-    const float *dstat = A.dens_stats;
+    const float *dstat = S.st;
     float g[D];
 #pragma unroll
     for (int d = 0; d < D; d++) g[d] = 0.0f;
@@ -722,7 +740,7 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
             if (q + stride + lane < r1) nx = __ldcs(A.rec + q + stride + lane);
             float gd[D];
             bool ad = false;
-            has = process_batch<D, DENS, NR, false, 1, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
+            has = process_batch<D, DENS, NR, true, 1, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
                                                                    dstat, part[warp]);
         }
         if (lane == 0) has_w[warp] = has;
@@ -740,7 +758,7 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
         __syncthreads();
     }
     if (warp != 0 || !valid) return;
-    finish_node<D, false>(A, node, ys, g, act);
+    finish_node<D, true>(A, node, ys, g, act);
 }
 
 // Position of the k-th set bit (k from 0) of m, which has more than k set
@@ -787,13 +805,13 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
 #endif
     const uint32_t w0 = sbeg >> 5, nw = send > sbeg ? ((send - 1) >> 5) - w0 + 1 : 0;
     if (nw > kSplitWords) {  // block-uniform
-        if (warp == 0) epoch_segment<D, DENS, NR, false, kU, FAST, false, true>(A, S, node0, lane);
+        if (warp == 0) epoch_segment<D, DENS, NR, true, kU, FAST, false, true>(A, S, node0, lane);
         return;
     }
     const uint32_t node = node0 + lane;
     const bool valid = node < A.n;
     float ys[D];
-    if (warp == 0) load_segment<D, DENS, false>(A, S, node0, lane, ys);
+    if (warp == 0) load_segment<D, DENS, true>(A, S, node0, lane, ys);
     // masked words and their popcounts; exclusive prefix by warp 0
     for (uint32_t t = threadIdx.x; t < nw; t += blockDim.x) {
         const uint32_t wi = w0 + t;
@@ -821,7 +839,7 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
     }
     __syncthreads();
     const uint32_t total = pre[kSplitWords];
-    const float *dstat = A.dens_stats;
+    const float *dstat = S.st;
     float g[D];
 #pragma unroll
     for (int d = 0; d < D; d++) g[d] = 0.0f;
@@ -847,7 +865,7 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
             }
             float gd[D];
             bool ad = false;
-            has = process_batch<D, DENS, NR, false, kU, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
+            has = process_batch<D, DENS, NR, true, kU, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
                                                                     dstat, part[warp]);
         }
         if (lane == 0) has_w[warp] = has;
@@ -865,7 +883,7 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
         __syncthreads();
     }
     if (warp != 0 || !valid) return;
-    finish_node<D, false>(A, node, ys, g, act);
+    finish_node<D, true>(A, node, ys, g, act);
 }
 
 }  // namespace umapcu

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kWarps * 32, epoch_min_blocks<D, DENS, FAST>()
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t node0 = (blockIdx.x * kWarps + warp) * 32u;
     if (node0 >= A.n) return;
-    epoch_segment<D, DENS, NR, false, KU, FAST, LIST, BITS>(A, smem[warp], node0, lane);
+    epoch_segment<D, DENS, NR, true, KU, FAST, LIST, BITS>(A, smem[warp], node0, lane);
 }
 
 // Schedule lists on a problem too small to fill the GPU with one warp per
@@ -202,9 +202,11 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
     const uint32_t nc = min(node0, n);
     S.beg[lane] = A.offsets[valid ? node : n];
     if (lane == 31) S.beg[32] = A.offsets[min(nc + 32u, n)];
+    grid_wait();
+    grid_trigger();
     if (valid) {
         float ys[D];
-        load_row<D>(A.y, node, ys);
+        load_row<D, true>(A.y, node, ys);
 #pragma unroll
         for (int d = 0; d < D; d++) S.ys[lane][d] = ys[d];
     }
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
             in[u] = in[u] && checked_ok(o[u] < n, A.err);
 #pragma unroll
             for (int d = 0; d < D; d++) yo[u][d] = 0.0f;
-            if (in[u]) load_row_keep<D>(A.y, o[u], yo[u], pol);
+            if (in[u]) load_row_keep<D, true>(A.y, o[u], yo[u], pol);
         }
         // the next window's endpoints, in flight while this one computes
         if (w0 + kWin < seg_end)
@@ -434,6 +436,23 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
 // of the 148 SMs) the list path gives each segment a whole block.
 constexpr uint32_t kSplitSegments = 148 * 9;
 
+// A kernel of one argument block behind the stream's last one, whose end it
+// waits for itself (grid_wait).
+template <class Args>
+static void launch_after(void (*kernel)(Args), unsigned grid, unsigned threads, const Args &A, cudaStream_t s)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    check_cuda(cudaLaunchKernelEx(&cfg, kernel, A), "epoch launch");
+}
+
 template <int D, bool DENS>
 static void launch_epoch_t(const EpochArgs &A, cudaStream_t s)
 {
@@ -441,25 +460,25 @@ static void launch_epoch_t(const EpochArgs &A, cudaStream_t s)
     const bool fast = !A.injected && A.sampler == UMAPCU_NEG_REF_HASH && !A.precise_pow;
     const unsigned grid = ceil_div(nseg, kWarps);
     if (A.rec && nseg < kSplitSegments) {
-        if (A.neg_rate == 5 && fast) k_epoch_split<D, DENS, 5, true><<<nseg, kWarps * 32, 0, s>>>(A);
-        else if (A.neg_rate == 5) k_epoch_split<D, DENS, 5, false><<<nseg, kWarps * 32, 0, s>>>(A);
-        else k_epoch_split<D, DENS, 0, false><<<nseg, kWarps * 32, 0, s>>>(A);
+        if (A.neg_rate == 5 && fast) launch_after(k_epoch_split<D, DENS, 5, true>, nseg, kWarps * 32, A, s);
+        else if (A.neg_rate == 5) launch_after(k_epoch_split<D, DENS, 5, false>, nseg, kWarps * 32, A, s);
+        else launch_after(k_epoch_split<D, DENS, 0, false>, nseg, kWarps * 32, A, s);
     } else if (A.rec) {
-        if (A.neg_rate == 5 && fast) k_epoch<D, DENS, 5, true, true><<<grid, kWarps * 32, 0, s>>>(A);
-        else if (A.neg_rate == 5) k_epoch<D, DENS, 5, false, true><<<grid, kWarps * 32, 0, s>>>(A);
-        else k_epoch<D, DENS, 0, false, true><<<grid, kWarps * 32, 0, s>>>(A);
+        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true, true>, grid, kWarps * 32, A, s);
+        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5, false, true>, grid, kWarps * 32, A, s);
+        else launch_after(k_epoch<D, DENS, 0, false, true>, grid, kWarps * 32, A, s);
     } else if (A.bits && nseg < kSplitSegments) {
-        if (A.neg_rate == 5 && fast) k_epoch_split_bits<D, DENS, 5, true><<<nseg, kSplitBitsWarps * 32, 0, s>>>(A);
-        else if (A.neg_rate == 5) k_epoch_split_bits<D, DENS, 5, false><<<nseg, kSplitBitsWarps * 32, 0, s>>>(A);
-        else k_epoch_split_bits<D, DENS, 0, false><<<nseg, kSplitBitsWarps * 32, 0, s>>>(A);
+        if (A.neg_rate == 5 && fast) launch_after(k_epoch_split_bits<D, DENS, 5, true>, nseg, kSplitBitsWarps * 32, A, s);
+        else if (A.neg_rate == 5) launch_after(k_epoch_split_bits<D, DENS, 5, false>, nseg, kSplitBitsWarps * 32, A, s);
+        else launch_after(k_epoch_split_bits<D, DENS, 0, false>, nseg, kSplitBitsWarps * 32, A, s);
     } else if (A.bits) {
-        if (A.neg_rate == 5 && fast) k_epoch<D, DENS, 5, true, false, true><<<grid, kWarps * 32, 0, s>>>(A);
-        else if (A.neg_rate == 5) k_epoch<D, DENS, 5, false, false, true><<<grid, kWarps * 32, 0, s>>>(A);
-        else k_epoch<D, DENS, 0, false, false, true><<<grid, kWarps * 32, 0, s>>>(A);
+        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true, false, true>, grid, kWarps * 32, A, s);
+        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5, false, false, true>, grid, kWarps * 32, A, s);
+        else launch_after(k_epoch<D, DENS, 0, false, false, true>, grid, kWarps * 32, A, s);
     } else {
-        if (A.neg_rate == 5 && fast) k_epoch<D, DENS, 5, true><<<grid, kWarps * 32, 0, s>>>(A);
-        else if (A.neg_rate == 5) k_epoch<D, DENS, 5><<<grid, kWarps * 32, 0, s>>>(A);
-        else k_epoch<D, DENS, 0><<<grid, kWarps * 32, 0, s>>>(A);
+        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true>, grid, kWarps * 32, A, s);
+        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5>, grid, kWarps * 32, A, s);
+        else launch_after(k_epoch<D, DENS, 0>, grid, kWarps * 32, A, s);
     }
 }
 
@@ -484,8 +503,8 @@ void launch_dens_update(const DensArgs &Dn, uint32_t n_dim, cudaStream_t s)
     const uint32_t nb = ceil_div(Dn.n, kDensBlock);
 #define UMAPCU_CASE(DD)                                                   \
     case DD:                                                              \
-        if (Dn.precise_pow) k_dens_update<DD, true><<<nb, kDensBlock, 0, s>>>(Dn); \
-        else k_dens_update<DD, false><<<nb, kDensBlock, 0, s>>>(Dn);       \
+        if (Dn.precise_pow) launch_after(k_dens_update<DD, true>, nb, kDensBlock, Dn, s); \
+        else launch_after(k_dens_update<DD, false>, nb, kDensBlock, Dn, s); \
         break;
     switch (n_dim) {
         UMAPCU_CASE(1) UMAPCU_CASE(2) UMAPCU_CASE(3) UMAPCU_CASE(4)
