@@ -25,9 +25,12 @@ namespace {
 
 constexpr size_t kChunk = (size_t)1 << 20;
 constexpr unsigned kMaxThreads = 8;
-// Copies below this gain nothing over the runtime's (starting the threads takes
-// about 0.1 ms, a copy of 2 MB 0.25).
-constexpr size_t kLeast = (size_t)4 << 20;
+// Copies below these gain nothing over the runtime's: starting the threads takes
+// 0.1-0.2 ms. Up, from touched pages: 4 MB 0.24 (the runtime) and 0.26 ms, 8 MB
+// 0.45 and 0.42, 16 MB 0.83 and 0.62. Down into touched pages, as the allocator
+// hands them out again: 6 MB 0.46 and 0.54, 16 MB 1.18 and 1.08, 32 MB 2.3 and
+// 1.5; into fresh ones 8 MB 1.7 and 0.83, 32 MB 6.6 and 1.8.
+constexpr size_t kLeastUp = (size_t)8 << 20, kLeastDown = (size_t)16 << 20;
 
 std::mutex g_mu;
 uint8_t *g_block = nullptr;  // the idle block; null while taken or not allocated
@@ -128,7 +131,7 @@ cudaError_t move_chunks(uint8_t *dst, const uint8_t *src, size_t bytes, bool to_
 
 bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaStream_t s)
 {
-    if (bytes < kLeast || copy_threads() < 2) return false;
+    if (bytes < (to_device ? kLeastUp : kLeastDown) || copy_threads() < 2) return false;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, to_device ? src : dst) != cudaSuccess) {
         cudaGetLastError();

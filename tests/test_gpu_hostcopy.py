@@ -21,9 +21,10 @@ def _by_parts(d):
     return [np.concatenate([p[t] for p in parts]) for t in range(2)]
 
 
-# 4 MiB is the least such copy, a chunk 1 MiB: rows of 4 k bytes up and 4 bytes
-# a row down, at the least size, one short of it, and with odd remainders
-@pytest.mark.parametrize("n,k", [(262_143, 4), (262_144, 4), (262_145, 4), (1_048_577, 1), (1_500_007, 3)])
+# 8 MiB up and 16 MiB down are the least such copies, a chunk 1 MiB: rows of 4 k
+# bytes up and 4 bytes a row down, at the least sizes, one short of them, and
+# with odd remainders
+@pytest.mark.parametrize("n,k", [(524_287, 4), (524_288, 4), (524_289, 4), (4_194_303, 1), (4_194_304, 1), (4_500_007, 1)])
 def test_large_copies_equal_small_ones(n, k):
     d = _rows(n, k, n)
     sigma, rho = umapcu.smooth_knn_dist(d)
@@ -32,7 +33,7 @@ def test_large_copies_equal_small_ones(n, k):
 
 
 def test_large_copies_from_several_threads():
-    data = [_rows(1_200_000 + i, 2, i) for i in range(4)]
+    data = [_rows(4_300_000 + i, 1, i) for i in range(4)]
     got = [None] * 4
 
     def work(i):
