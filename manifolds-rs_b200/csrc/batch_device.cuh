@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_persistent(const Batch
                 sargs[warp] = A;
             }
             __syncwarp();
-            epoch_segment<D, false, NR, true, KU, FAST, false, BITS>(sargs[warp], smem[warp], (s - P.seg_base) * 32u,
+            epoch_segment<D, false, NR, kShared, KU, FAST, false, BITS>(sargs[warp], smem[warp], (s - P.seg_base) * 32u,
                                                                      lane);
         }
         __threadfence();
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_persistent(const Batch
 // One launch per epoch, each overlapping the one before as the single-problem
 // kernels do (grid_wait in load_segment). The fast two-dimensional form runs at
 // ten blocks an SM with half-word pieces, like theirs: 48 problems of 0.5-20k
-// points, 100 epochs, whole run @BATCH.
+// points, 100 epochs: 4.07 ms on the device either way (the gathers bound it).
 template <int D, int NR, bool FAST, bool BITS>
 constexpr bool batch_dense() { return FAST && BITS && D == 2 && NR == 5; }
 template <int D, int NR, int KU, bool FAST = false, bool BITS = false>
@@ -154,10 +154,12 @@ __global__ void __launch_bounds__(kWarps * 32, batch_dense<D, NR, FAST, BITS>() 
         sargs[warp] = A;
     }
     __syncwarp();
-    epoch_segment<D, false, NR, true, KU, FAST, false, BITS, BP>(sargs[warp], smem[warp], (s - P.seg_base) * 32u, lane);
+    epoch_segment<D, false, NR, kDependent, KU, FAST, false, BITS, BP>(sargs[warp], smem[warp], (s - P.seg_base) * 32u, lane);
 }
 
-// k_batch_epoch behind the stream's last kernel, whose end it waits for itself.
+// k_batch_epoch behind the stream's last kernel, whose end it waits for itself
+// -- unless the grid fits the device but not beside the one before it, whose
+// leftovers its blocks would then be packed onto (epoch_form in layout.cu).
 inline void launch_batch_epoch(void (*kernel)(BatchArgs, uint32_t), unsigned grid, const BatchArgs &B, uint32_t e,
                                cudaStream_t s)
 {
@@ -169,7 +171,8 @@ inline void launch_batch_epoch(void (*kernel)(BatchArgs, uint32_t), unsigned gri
     cfg.blockDim = dim3(kWarps * 32);
     cfg.stream = s;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    const unsigned slots = 8u * (unsigned)device_sm_count();
+    cfg.numAttrs = 2 * grid <= slots || grid > slots ? 1 : 0;
     check_cuda(cudaLaunchKernelEx(&cfg, kernel, B, e), "k_batch_epoch");
 }
 

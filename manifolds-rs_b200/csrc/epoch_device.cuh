@@ -109,17 +109,24 @@ __device__ __forceinline__ uint64_t l2_keep_policy()
     return pol;
 }
 
-// COH = true: loads of data that other SMs rewrite while the kernel runs
-// (the epoch kernels, which overlap the previous epoch's, and the persistent
-// multi-problem kernel: the embedding buffers, moments and cursors change
-// roles every epoch). They go through L2 (ld.global.cg)
-// instead of the non-coherent read-only path / L1.
-template <int D, bool COH = false>
+// How embedding buffers, moments and cursors are read; they change roles every
+// epoch. kStatic: nothing writes them while the kernel runs, the non-coherent
+// path. kDependent: the previous epoch's kernel may still run when this one
+// starts (grid_wait): coherent loads that keep nothing in L1. kShared: other SMs
+// rewrite them during the kernel (the persistent multi-problem kernel): through
+// L2 (ld.global.cg), also the gathers, which that makes 3 % slower (160k points
+// 24.6 -> 25.3 us an epoch).
+enum { kStatic = 0, kDependent = 1, kShared = 2 };
+template <int D, int COH = kStatic>
 __device__ __forceinline__ void load_row_keep(const float *__restrict__ y, uint32_t i, float (&out)[D], uint64_t pol)
 {
     if constexpr (D == 2) {
         const float *a = y + 2ull * i;
-        if constexpr (COH)
+        if constexpr (COH == kDependent)
+            asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+                         : "=f"(out[0]), "=f"(out[1])
+                         : "l"(a), "l"(pol));
+        else if constexpr (COH == kShared)
             asm volatile("ld.global.cg.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
                          : "=f"(out[0]), "=f"(out[1])
                          : "l"(a), "l"(pol));
@@ -129,7 +136,11 @@ __device__ __forceinline__ void load_row_keep(const float *__restrict__ y, uint3
                          : "l"(a), "l"(pol));
     } else if constexpr (D == 4) {
         const float *a = y + 4ull * i;
-        if constexpr (COH)
+        if constexpr (COH == kDependent)
+            asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                         : "=f"(out[0]), "=f"(out[1]), "=f"(out[2]), "=f"(out[3])
+                         : "l"(a), "l"(pol));
+        else if constexpr (COH == kShared)
             asm volatile("ld.global.cg.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
                          : "=f"(out[0]), "=f"(out[1]), "=f"(out[2]), "=f"(out[3])
                          : "l"(a), "l"(pol));
@@ -141,7 +152,9 @@ __device__ __forceinline__ void load_row_keep(const float *__restrict__ y, uint3
 #pragma unroll
         for (int d = 0; d < D; d++) {
             const float *a = y + (uint64_t)i * D + d;
-            if constexpr (COH)
+            if constexpr (COH == kDependent)
+                asm volatile("ld.global.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(out[d]) : "l"(a), "l"(pol));
+            else if constexpr (COH == kShared)
                 asm volatile("ld.global.cg.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(out[d]) : "l"(a), "l"(pol));
             else
                 asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(out[d]) : "l"(a), "l"(pol));
@@ -149,7 +162,7 @@ __device__ __forceinline__ void load_row_keep(const float *__restrict__ y, uint3
     }
 }
 
-template <int D, bool COH = false>
+template <int D, int COH = kStatic>
 __device__ __forceinline__ void load_row(const float *__restrict__ y, uint32_t i, float (&out)[D])
 {
     if constexpr (D == 2) {
@@ -279,7 +292,7 @@ struct BatchRows {
 // The batch's per-node sums go to part[j] for the nodes in the returned
 // mask; unless SPLIT, the node's lane then adds them to g (and sets act).
 // PRE: the entry's negatives and all its rows come in pre (FAST, NR > 0 only).
-template <int D, bool DENS, int NR, bool COH, int KU, bool FAST, bool SPLIT = false, bool PRE = false,
+template <int D, bool DENS, int NR, int COH, int KU, bool FAST, bool SPLIT = false, bool PRE = false,
           class Smem = WarpSmem<D, KU>>
 __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, bool live, uint32_t p,
                                                   uint32_t o, uint32_t j, uint32_t edge_local, uint32_t node0,
@@ -463,15 +476,17 @@ __device__ __forceinline__ unsigned process_batch(const EpochArgs &A, Smem &S, b
 
 // The segment's row starts, positions (and densMAP node data) into shared
 // memory; ys = the lane's node's position (zeros beyond n).
-template <int D, bool DENS, bool COH, class Smem>
+template <int D, bool DENS, int COH, class Smem>
 __device__ __forceinline__ void load_segment(const EpochArgs &A, Smem &S, uint32_t node0, int lane, float (&ys)[D])
 {
     const uint32_t node = node0 + lane;
     const bool valid = node < A.n;
     S.beg[lane] = A.offsets[valid ? node : A.n];
     if (lane == 31) S.beg[32] = A.offsets[min(node0 + 32u, A.n)];
-    grid_wait();  // the positions, moments and cursors are the previous epoch's
-    grid_trigger();
+    if constexpr (COH == kDependent) {
+        grid_wait();  // the positions, moments and cursors are the previous epoch's
+        grid_trigger();
+    }
     if (valid) load_row<D, COH>(A.y_cur, node, ys);
     else {
 #pragma unroll
@@ -500,7 +515,7 @@ __device__ __forceinline__ void load_segment(const EpochArgs &A, Smem &S, uint32
 
 // The node's step (umap_adam_update, umap_optimiser_gpu.rs:887-923, or the
 // SGD step) from its gradient g, and the next embedding buffer's row.
-template <int D, bool COH>
+template <int D, int COH>
 __device__ __forceinline__ void finish_node(const EpochArgs &A, uint32_t node, const float (&ys)[D],
                                             const float (&g)[D], bool act)
 {
@@ -533,7 +548,7 @@ __device__ __forceinline__ void finish_node(const EpochArgs &A, uint32_t node, c
 // (A.rec / A.seg_ptr) instead of a scan of its CSR range.
 // BITS: the scan reads the epoch's active-entry bitmask (A.bits) in place of
 // the entries' (cursor, period) and writes no cursor.
-template <int D, bool DENS, int NR, bool COH, int KU = kU, bool FAST = false, bool LIST = false,
+template <int D, bool DENS, int NR, int COH, int KU = kU, bool FAST = false, bool LIST = false,
           bool BITS = false, int BP = 32>
 __device__ __forceinline__ void epoch_segment(const EpochArgs &A, WarpSmem<D, KU, BITS, DENS, BP> &S, uint32_t node0,
                                               int lane)
@@ -700,14 +715,14 @@ __device__ __forceinline__ void epoch_segment(const EpochArgs &A, WarpSmem<D, KU
     finish_node<D, COH>(A, node, ys, g, act);
 }
 
-// One epoch of one 32-node segment run by all kWarps warps of a block, for
-// problems too small to fill the GPU with one warp per segment (schedule
+// One epoch of one 32-node segment run by all W warps of a block, for
+// problems that do not fill the GPU evenly with one warp per segment (schedule
 // lists only). The segment's batches are the same 32-record slices of its
 // list as in epoch_segment; in each round warp w evaluates batch
-// round * kWarps + w into its own part[w], and warp 0's node lanes add the
+// round * W + w into its own part[w], and warp 0's node lanes add the
 // round's partials in batch order -- the order epoch_segment adds them in, so
 // the result is bit-identical.
-template <int D, bool DENS, int NR, bool FAST>
+template <int D, bool DENS, int NR, bool FAST, int W>
 __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem<D, 1, false, DENS> &S,
                                                     float (*part)[32][D],
                                                     unsigned *has_w, uint32_t node0, int warp, int lane)
@@ -715,7 +730,7 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
     const uint32_t node = node0 + lane;
     const bool valid = node < A.n;
     float ys[D];
-    if (warp == 0) load_segment<D, DENS, true>(A, S, node0, lane, ys);
+    if (warp == 0) load_segment<D, DENS, kDependent>(A, S, node0, lane, ys);
     __syncthreads();
     const float *dstat = S.st;
     float g[D];
@@ -724,7 +739,7 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
     bool act = false;
     const uint32_t sg = node0 >> 5;
     const uint64_t r0 = A.seg_ptr[A.seg_unit[sg]], r1 = A.seg_ptr[A.seg_unit[sg + 1]];
-    const uint64_t stride = 32u * kWarps;
+    const uint64_t stride = 32u * W;
     uint2 nx = make_uint2(0, 0);
     if (r0 + 32u * warp + lane < r1) nx = __ldcs(A.rec + r0 + 32u * warp + lane);
     for (uint64_t q0 = r0; q0 < r1; q0 += stride) {  // block-uniform
@@ -740,14 +755,14 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
             if (q + stride + lane < r1) nx = __ldcs(A.rec + q + stride + lane);
             float gd[D];
             bool ad = false;
-            has = process_batch<D, DENS, NR, true, 1, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
+            has = process_batch<D, DENS, NR, kDependent, 1, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
                                                                    dstat, part[warp]);
         }
         if (lane == 0) has_w[warp] = has;
         __syncthreads();
         if (warp == 0) {
 #pragma unroll
-            for (int w = 0; w < kWarps; w++) {
+            for (int w = 0; w < W; w++) {
                 if ((has_w[w] >> lane) & 1u) {
                     act = true;
 #pragma unroll
@@ -758,7 +773,7 @@ __device__ __forceinline__ void epoch_segment_split(const EpochArgs &A, WarpSmem
         __syncthreads();
     }
     if (warp != 0 || !valid) return;
-    finish_node<D, true>(A, node, ys, g, act);
+    finish_node<D, kDependent>(A, node, ys, g, act);
 }
 
 // Position of the k-th set bit (k from 0) of m, which has more than k set
@@ -781,11 +796,6 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t k)
 // Words of a segment's bitmask one block of epoch_segment_split_bits holds;
 // a longer segment runs on warp 0 alone with the sequential scan.
 constexpr uint32_t kSplitWords = 256;
-// Warps of a k_epoch_split_bits block: a small problem's segment has a few
-// batches per epoch, and each warp takes one batch per round, so more warps
-// mean fewer dependent rounds of gathers per epoch.
-constexpr int kSplitBitsWarps = 8;
-
 // The bitmask form of epoch_segment_split: the block reads the segment's
 // words of the epoch's bitmask, masks them to the segment's entries, and
 // forms prefix counts; batch b is then the active entries of rank 32 b ..
@@ -793,7 +803,7 @@ constexpr int kSplitBitsWarps = 8;
 // lane t finds its entry by searching the prefix counts and selecting the
 // bit. Partials are added in batch order as in epoch_segment_split, so the
 // result is bit-identical to the scan.
-template <int D, bool DENS, int NR, bool FAST, int W = kWarps>
+template <int D, bool DENS, int NR, bool FAST, int W>
 __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, WarpSmem<D, kU, true, DENS, 32> &S,
                                                          float (*part)[32][D],
                                                          unsigned *has_w, uint32_t *wm, uint32_t *pre,
@@ -805,13 +815,13 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
 #endif
     const uint32_t w0 = sbeg >> 5, nw = send > sbeg ? ((send - 1) >> 5) - w0 + 1 : 0;
     if (nw > kSplitWords) {  // block-uniform
-        if (warp == 0) epoch_segment<D, DENS, NR, true, kU, FAST, false, true>(A, S, node0, lane);
+        if (warp == 0) epoch_segment<D, DENS, NR, kDependent, kU, FAST, false, true>(A, S, node0, lane);
         return;
     }
     const uint32_t node = node0 + lane;
     const bool valid = node < A.n;
     float ys[D];
-    if (warp == 0) load_segment<D, DENS, true>(A, S, node0, lane, ys);
+    if (warp == 0) load_segment<D, DENS, kDependent>(A, S, node0, lane, ys);
     // masked words and their popcounts; exclusive prefix by warp 0
     for (uint32_t t = threadIdx.x; t < nw; t += blockDim.x) {
         const uint32_t wi = w0 + t;
@@ -865,7 +875,7 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
             }
             float gd[D];
             bool ad = false;
-            has = process_batch<D, DENS, NR, true, kU, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
+            has = process_batch<D, DENS, NR, kDependent, kU, FAST, true>(A, S, live, p, o, j, el, node0, lane, gd, ad,
                                                                     dstat, part[warp]);
         }
         if (lane == 0) has_w[warp] = has;
@@ -883,7 +893,7 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
         __syncthreads();
     }
     if (warp != 0 || !valid) return;
-    finish_node<D, true>(A, node, ys, g, act);
+    finish_node<D, kDependent>(A, node, ys, g, act);
 }
 
 }  // namespace umapcu

@@ -56,7 +56,8 @@ constexpr int epoch_min_blocks() { return FAST && !DENS && D <= 2 ? 10 : 6; }
 template <int D, bool DENS, bool FAST>
 constexpr int bits_piece() { return FAST && !DENS && D <= 2 ? 16 : 32; }
 
-template <int D, bool DENS, int NR, bool FAST = false, bool LIST = false, bool BITS = false>
+// PLAIN: for launches after the end of the previous kernel.
+template <int D, bool DENS, int NR, bool FAST = false, bool LIST = false, bool BITS = false, bool PLAIN = false>
 __global__ void __launch_bounds__(kWarps * 32, epoch_min_blocks<D, DENS, FAST>()) k_epoch(const EpochArgs A)
 {
     constexpr int KU = LIST ? 1 : kU;  // the list path keeps no scan queue
@@ -64,32 +65,32 @@ __global__ void __launch_bounds__(kWarps * 32, epoch_min_blocks<D, DENS, FAST>()
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t node0 = (blockIdx.x * kWarps + warp) * 32u;
     if (node0 >= A.n) return;
-    epoch_segment<D, DENS, NR, true, KU, FAST, LIST, BITS>(A, smem[warp], node0, lane);
+    epoch_segment<D, DENS, NR, PLAIN ? kStatic : kDependent, KU, FAST, LIST, BITS>(A, smem[warp], node0, lane);
 }
 
-// Schedule lists on a problem too small to fill the GPU with one warp per
-// segment: one block (kWarps warps) per segment, see epoch_segment_split.
-template <int D, bool DENS, int NR, bool FAST>
-__global__ void __launch_bounds__(kWarps * 32) k_epoch_split(const EpochArgs A)
+// Schedule lists with one block of W warps per segment, see
+// epoch_segment_split.
+template <int D, bool DENS, int NR, bool FAST, int W>
+__global__ void __launch_bounds__(W * 32) k_epoch_split(const EpochArgs A)
 {
     __shared__ WarpSmem<D, 1, false, DENS> seg;
-    __shared__ float part[kWarps][32][D];
-    __shared__ unsigned has_w[kWarps];
+    __shared__ float part[W][32][D];
+    __shared__ unsigned has_w[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    epoch_segment_split<D, DENS, NR, FAST>(A, seg, part, has_w, blockIdx.x * 32u, warp, lane);
+    epoch_segment_split<D, DENS, NR, FAST, W>(A, seg, part, has_w, blockIdx.x * 32u, warp, lane);
 }
 
-// The bitmask form on a small problem: one block per segment, see
+// The bitmask form with one block of W warps per segment, see
 // epoch_segment_split_bits.
-template <int D, bool DENS, int NR, bool FAST>
-__global__ void __launch_bounds__(kSplitBitsWarps * 32) k_epoch_split_bits(const EpochArgs A)
+template <int D, bool DENS, int NR, bool FAST, int W>
+__global__ void __launch_bounds__(W * 32) k_epoch_split_bits(const EpochArgs A)
 {
     __shared__ WarpSmem<D, kU, true, DENS> seg;
-    __shared__ float part[kSplitBitsWarps][32][D];
-    __shared__ unsigned has_w[kSplitBitsWarps];
+    __shared__ float part[W][32][D];
+    __shared__ unsigned has_w[W];
     __shared__ uint32_t wm[kSplitWords], pre[kSplitWords + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    epoch_segment_split_bits<D, DENS, NR, FAST, kSplitBitsWarps>(A, seg, part, has_w, wm, pre, blockIdx.x * 32u, warp, lane);
+    epoch_segment_split_bits<D, DENS, NR, FAST, W>(A, seg, part, has_w, wm, pre, blockIdx.x * 32u, warp, lane);
 }
 
 // ------------------------------------------------------------ densMAP
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
     grid_trigger();
     if (valid) {
         float ys[D];
-        load_row<D, true>(A.y, node, ys);
+        load_row<D, kDependent>(A.y, node, ys);
 #pragma unroll
         for (int d = 0; d < D; d++) S.ys[lane][d] = ys[d];
     }
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
             in[u] = in[u] && checked_ok(o[u] < n, A.err);
 #pragma unroll
             for (int d = 0; d < D; d++) yo[u][d] = 0.0f;
-            if (in[u]) load_row_keep<D, true>(A.y, o[u], yo[u], pol);
+            if (in[u]) load_row_keep<D, kDependent>(A.y, o[u], yo[u], pol);
         }
         // the next window's endpoints, in flight while this one computes
         if (w0 + kWin < seg_end)
@@ -432,14 +433,10 @@ __global__ void __launch_bounds__(kDensBlock) k_dens_update(const DensArgs A)
 
 // ------------------------------------------------------------ launchers
 
-// Below this many segments (about 9 blocks of one warp per segment on each
-// of the 148 SMs) the list path gives each segment a whole block.
-constexpr uint32_t kSplitSegments = 148 * 9;
-
-// A kernel of one argument block behind the stream's last one, whose end it
-// waits for itself (grid_wait).
+// A kernel of one argument block on the stream; dependent: launched behind the
+// stream's last kernel, whose end it waits for itself (grid_wait).
 template <class Args>
-static void launch_after(void (*kernel)(Args), unsigned grid, unsigned threads, const Args &A, cudaStream_t s)
+static void launch_one(void (*kernel)(Args), unsigned grid, unsigned threads, const Args &A, bool dependent, cudaStream_t s)
 {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -449,8 +446,72 @@ static void launch_after(void (*kernel)(Args), unsigned grid, unsigned threads, 
     cfg.blockDim = dim3(threads);
     cfg.stream = s;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     check_cuda(cudaLaunchKernelEx(&cfg, kernel, A), "epoch launch");
+}
+
+// Below this many segments (about 9 blocks of one warp per segment on each
+// of the 148 SMs) a segment gets a whole block in every configuration.
+constexpr uint32_t kSplitSegments = 148 * 9;
+
+// How an epoch is launched: `warps` per segment in a block of its own, or 0 for
+// k_epoch (a warp per segment); dependent on the kernel before or after its end.
+struct EpochForm {
+    int warps;
+    bool dependent;
+    bool plain() const { return !warps && !dependent; }
+};
+
+// The form by the number of segments; P is how many warps of k_epoch the device
+// holds at once. us an epoch, fast configuration, k = 15, two dimensions unless
+// said otherwise (k_epoch is the warp per segment, launched dependent):
+//  * few segments are bound by the latency of their batches: eight warps with
+//    bitmasks (20k points: 8 warps 7.6, 6 9.0, 3 8.1), six up to a third of P
+//    (42k: 6 10.9, 8 11.5, k_epoch 11.6; 60k: 13.1, k_epoch 13.8), in three
+//    dimensions up to half (50k: 21.9, k_epoch 23.4). Lists need no ranks and
+//    take six up to 444 segments (10k: 5.5, four 6.3) and three up to 1000 (30k:
+//    7.9, six 9.1), in three dimensions six up to half of P (50k: 20.8, k_epoch
+//    22.6). With the density term eight (bitmasks) or four (lists).
+//  * up to half of P: k_epoch, dependent.
+//  * between P / 2 and P a dependent grid does not fit beside the one before
+//    it, its first blocks are packed onto what is left of the SMs and the epoch
+//    takes a third longer (100k points 24.9 us, launched after 18.8); just above
+//    P the last few warps make a round of their own. Blocks of three warps a
+//    segment spread evenly: 100k 17.5, 200k 29.8 (k_epoch 31.7), 200k in three
+//    dimensions 68 (72), 200k densMAP 53 (55.6), up to 1.27 P in two dimensions
+//    (250k: 35.8, k_epoch 35.7) and 2 P in the kernels of six blocks an SM;
+//    from 0.78 P (with the density term from P / 2) to P k_epoch launched after
+//    its predecessor is as good in two dimensions (160k: 24.3, three warps
+//    25.0; 70k densMAP, k = 30: 26.4 and 27.6).
+//  * beyond: k_epoch, dependent (1M 112.7, launched after 114.5).
+template <int D, bool DENS>
+static EpochForm epoch_form(uint32_t nseg, bool lists, bool fast5)
+{
+    if (!fast5) {
+        const uint32_t P = epoch_min_blocks<D, DENS, false>() * kWarps * (uint32_t)device_sm_count();
+        if (nseg < kSplitSegments) return {lists ? 4 : 8, true};
+        return {0, 2 * nseg <= P || nseg > P};
+    }
+    const uint32_t P = epoch_min_blocks<D, DENS, true>() * kWarps * (uint32_t)device_sm_count();
+    if (DENS) {
+        if (nseg < kSplitSegments) return {lists ? 4 : 8, true};
+    } else if (D > 2) {
+        if (lists || nseg >= 700) {
+            if (2 * nseg <= P) return {6, true};
+        } else {
+            return {8, true};
+        }
+    } else if (lists) {
+        if (nseg <= 444) return {6, true};
+        if (nseg <= 1000) return {3, true};
+    } else {
+        if (nseg < 700) return {8, true};
+        if (3 * nseg <= P) return {6, true};
+    }
+    if (2 * nseg <= P) return {0, true};
+    if (D <= 2 && nseg <= P && (DENS || nseg > P / 100 * 78)) return {0, false};
+    if (nseg <= (D <= 2 && !DENS ? P / 100 * 127 : 2 * P)) return {3, true};
+    return {0, true};
 }
 
 template <int D, bool DENS>
@@ -458,27 +519,40 @@ static void launch_epoch_t(const EpochArgs &A, cudaStream_t s)
 {
     const uint32_t nseg = ceil_div(A.n, 32);
     const bool fast = !A.injected && A.sampler == UMAPCU_NEG_REF_HASH && !A.precise_pow;
+    const bool fast5 = fast && A.neg_rate == 5;
     const unsigned grid = ceil_div(nseg, kWarps);
-    if (A.rec && nseg < kSplitSegments) {
-        if (A.neg_rate == 5 && fast) launch_after(k_epoch_split<D, DENS, 5, true>, nseg, kWarps * 32, A, s);
-        else if (A.neg_rate == 5) launch_after(k_epoch_split<D, DENS, 5, false>, nseg, kWarps * 32, A, s);
-        else launch_after(k_epoch_split<D, DENS, 0, false>, nseg, kWarps * 32, A, s);
+    const EpochForm f = epoch_form<D, DENS>(nseg, A.rec != nullptr, fast5);
+    if (f.warps && A.rec) {
+        if (fast5 && f.warps == 3) launch_one(k_epoch_split<D, DENS, 5, true, 3>, nseg, 96, A, f.dependent, s);
+        else if (fast5 && f.warps == 6) launch_one(k_epoch_split<D, DENS, 5, true, 6>, nseg, 192, A, f.dependent, s);
+        else if (fast5) launch_one(k_epoch_split<D, DENS, 5, true, 4>, nseg, 128, A, f.dependent, s);
+        else if (A.neg_rate == 5) launch_one(k_epoch_split<D, DENS, 5, false, 4>, nseg, 128, A, f.dependent, s);
+        else launch_one(k_epoch_split<D, DENS, 0, false, 4>, nseg, 128, A, f.dependent, s);
+    } else if (f.warps && A.bits) {
+        if (fast5 && f.warps == 3) launch_one(k_epoch_split_bits<D, DENS, 5, true, 3>, nseg, 96, A, f.dependent, s);
+        else if (fast5 && f.warps == 6) launch_one(k_epoch_split_bits<D, DENS, 5, true, 6>, nseg, 192, A, f.dependent, s);
+        else if (fast5) launch_one(k_epoch_split_bits<D, DENS, 5, true, 8>, nseg, 256, A, f.dependent, s);
+        else if (A.neg_rate == 5) launch_one(k_epoch_split_bits<D, DENS, 5, false, 8>, nseg, 256, A, f.dependent, s);
+        else launch_one(k_epoch_split_bits<D, DENS, 0, false, 8>, nseg, 256, A, f.dependent, s);
+    } else if (f.plain() && fast5 && D <= 2 && (A.rec || A.bits)) {
+        if constexpr (D <= 2) {
+            if (A.rec) launch_one(k_epoch<D, DENS, 5, true, true, false, true>, grid, kWarps * 32, A, false, s);
+            else launch_one(k_epoch<D, DENS, 5, true, false, true, true>, grid, kWarps * 32, A, false, s);
+        }
     } else if (A.rec) {
-        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true, true>, grid, kWarps * 32, A, s);
-        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5, false, true>, grid, kWarps * 32, A, s);
-        else launch_after(k_epoch<D, DENS, 0, false, true>, grid, kWarps * 32, A, s);
-    } else if (A.bits && nseg < kSplitSegments) {
-        if (A.neg_rate == 5 && fast) launch_after(k_epoch_split_bits<D, DENS, 5, true>, nseg, kSplitBitsWarps * 32, A, s);
-        else if (A.neg_rate == 5) launch_after(k_epoch_split_bits<D, DENS, 5, false>, nseg, kSplitBitsWarps * 32, A, s);
-        else launch_after(k_epoch_split_bits<D, DENS, 0, false>, nseg, kSplitBitsWarps * 32, A, s);
+        if (fast5) launch_one(k_epoch<D, DENS, 5, true, true>, grid, kWarps * 32, A, f.dependent, s);
+        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5, false, true>, grid, kWarps * 32, A, f.dependent, s);
+        else launch_one(k_epoch<D, DENS, 0, false, true>, grid, kWarps * 32, A, f.dependent, s);
     } else if (A.bits) {
-        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true, false, true>, grid, kWarps * 32, A, s);
-        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5, false, false, true>, grid, kWarps * 32, A, s);
-        else launch_after(k_epoch<D, DENS, 0, false, false, true>, grid, kWarps * 32, A, s);
+        if (fast5) launch_one(k_epoch<D, DENS, 5, true, false, true>, grid, kWarps * 32, A, f.dependent, s);
+        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5, false, false, true>, grid, kWarps * 32, A, f.dependent, s);
+        else launch_one(k_epoch<D, DENS, 0, false, false, true>, grid, kWarps * 32, A, f.dependent, s);
     } else {
-        if (A.neg_rate == 5 && fast) launch_after(k_epoch<D, DENS, 5, true>, grid, kWarps * 32, A, s);
-        else if (A.neg_rate == 5) launch_after(k_epoch<D, DENS, 5>, grid, kWarps * 32, A, s);
-        else launch_after(k_epoch<D, DENS, 0>, grid, kWarps * 32, A, s);
+        const uint32_t P = epoch_min_blocks<D, DENS, false>() * kWarps * (uint32_t)device_sm_count();
+        const bool dependent = 2 * nseg <= P || nseg > 2 * P;
+        if (fast5) launch_one(k_epoch<D, DENS, 5, true>, grid, kWarps * 32, A, dependent, s);
+        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5>, grid, kWarps * 32, A, dependent, s);
+        else launch_one(k_epoch<D, DENS, 0>, grid, kWarps * 32, A, dependent, s);
     }
 }
 
@@ -501,10 +575,14 @@ void launch_epoch(const EpochArgs &A, uint32_t n_dim, bool dens, cudaStream_t s)
 void launch_dens_update(const DensArgs &Dn, uint32_t n_dim, cudaStream_t s)
 {
     const uint32_t nb = ceil_div(Dn.n, kDensBlock);
+    // Dependent where the grid fits beside the epoch kernel before it, or is
+    // larger than the device (epoch_form)
+    const uint32_t slots = 8u * (uint32_t)device_sm_count();
+    const bool dependent = 2 * nb <= slots || nb > slots;
 #define UMAPCU_CASE(DD)                                                   \
     case DD:                                                              \
-        if (Dn.precise_pow) launch_after(k_dens_update<DD, true>, nb, kDensBlock, Dn, s); \
-        else launch_after(k_dens_update<DD, false>, nb, kDensBlock, Dn, s); \
+        if (Dn.precise_pow) launch_one(k_dens_update<DD, true>, nb, kDensBlock, Dn, dependent, s); \
+        else launch_one(k_dens_update<DD, false>, nb, kDensBlock, Dn, dependent, s); \
         break;
     switch (n_dim) {
         UMAPCU_CASE(1) UMAPCU_CASE(2) UMAPCU_CASE(3) UMAPCU_CASE(4)

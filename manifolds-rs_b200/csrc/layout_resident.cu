@@ -155,10 +155,10 @@ __global__ void __launch_bounds__(32 * (NG * G + 1), MIN_BLOCKS)
 #pragma unroll
     for (int d = 0; d < D; d++) ys[d] = m[d] = v[d] = 0.0f;
     if (warp == 0) {
-        load_segment<D, false, true>(A, S, node0, lane, ys);
+        load_segment<D, false, kShared>(A, S, node0, lane, ys);
         if (valid) {
-            load_row<D, true>(A.m, node, m);
-            load_row<D, true>(A.v, node, v);
+            load_row<D, kShared>(A.m, node, m);
+            load_row<D, kShared>(A.v, node, v);
             store_tagged<D>(ring + node, ys, 1u);
         }
     }
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(32 * (NG * G + 1), MIN_BLOCKS)
                 float gd[D];
                 bool ad = false;
                 // (the rows came after warp 0 had read the group's last sums)
-                const unsigned has = process_batch<D, false, NR, true, kU, true, true, true>(
+                const unsigned has = process_batch<D, false, NR, kShared, kU, true, true, true>(
                     A, S, live, 0u, o, j, el, node0, lane, gd, ad, nullptr, part[grp][mine], &R);
                 if (lane == 0) has_w[grp][mine] = has;
             }
