@@ -129,18 +129,14 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_persistent(const Batch
     }
 }
 
-// One launch per epoch, each overlapping the one before as the single-problem
-// kernels do (grid_wait in load_segment). The fast two-dimensional form runs at
-// ten blocks an SM with half-word pieces, like theirs: 48 problems of 0.5-20k
-// points, 100 epochs: 4.07 ms on the device either way (the gathers bound it).
-template <int D, int NR, bool FAST, bool BITS>
-constexpr bool batch_dense() { return FAST && BITS && D == 2 && NR == 5; }
-template <int D, int NR, int KU, bool FAST = false, bool BITS = false>
-__global__ void __launch_bounds__(kWarps * 32, batch_dense<D, NR, FAST, BITS>() ? 10 : 8)
-    k_batch_epoch(const BatchArgs B, uint32_t e)
+// One launch per epoch. DEPENDENT: overlapping the one before as the
+// single-problem kernels do (grid_wait in load_segment). Ten blocks an SM with
+// half-word pieces, as k_epoch has, spill here (the arguments come from shared
+// memory) and are 3 % slower.
+template <int D, int NR, int KU, bool FAST, bool BITS, bool DEPENDENT>
+__global__ void __launch_bounds__(kWarps * 32, 8) k_batch_epoch(const BatchArgs B, uint32_t e)
 {
-    constexpr int BP = batch_dense<D, NR, FAST, BITS>() ? 16 : 32;
-    __shared__ WarpSmem<D, KU, BITS, false, BP> smem[kWarps];
+    __shared__ WarpSmem<D, KU, BITS, false> smem[kWarps];
     __shared__ EpochArgs sargs[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t s = blockIdx.x * kWarps + warp;
@@ -154,15 +150,21 @@ __global__ void __launch_bounds__(kWarps * 32, batch_dense<D, NR, FAST, BITS>() 
         sargs[warp] = A;
     }
     __syncwarp();
-    epoch_segment<D, false, NR, kDependent, KU, FAST, false, BITS, BP>(sargs[warp], smem[warp], (s - P.seg_base) * 32u, lane);
+    epoch_segment<D, false, NR, DEPENDENT ? kDependent : kStatic, KU, FAST, false, BITS>(sargs[warp], smem[warp],
+                                                                                   (s - P.seg_base) * 32u, lane);
 }
 
-// k_batch_epoch behind the stream's last kernel, whose end it waits for itself
-// -- unless the grid fits the device but not beside the one before it, whose
-// leftovers its blocks would then be packed onto (epoch_form in layout.cu).
-inline void launch_batch_epoch(void (*kernel)(BatchArgs, uint32_t), unsigned grid, const BatchArgs &B, uint32_t e,
-                               cudaStream_t s)
+// Dependent unless the grid fits the device but not beside the one before it,
+// whose leftovers its blocks would then be packed onto (epoch_form in
+// layout.cu).
+template <int D, int NR, int KU, bool FAST, bool BITS>
+inline void launch_batch_epoch(const BatchArgs &B, uint32_t e, cudaStream_t s)
 {
+    const unsigned grid = ceil_div(B.n_segs, kWarps), slots = 8u * (unsigned)device_sm_count();
+    if (2 * grid > slots && grid <= slots) {
+        k_batch_epoch<D, NR, KU, FAST, BITS, false><<<grid, kWarps * 32, 0, s>>>(B, e);
+        return;
+    }
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -171,9 +173,8 @@ inline void launch_batch_epoch(void (*kernel)(BatchArgs, uint32_t), unsigned gri
     cfg.blockDim = dim3(kWarps * 32);
     cfg.stream = s;
     cfg.attrs = &attr;
-    const unsigned slots = 8u * (unsigned)device_sm_count();
-    cfg.numAttrs = 2 * grid <= slots || grid > slots ? 1 : 0;
-    check_cuda(cudaLaunchKernelEx(&cfg, kernel, B, e), "k_batch_epoch");
+    cfg.numAttrs = 1;
+    check_cuda(cudaLaunchKernelEx(&cfg, k_batch_epoch<D, NR, KU, FAST, BITS, true>, B, e), "k_batch_epoch");
 }
 
 struct BatchConfig {
@@ -193,9 +194,8 @@ inline void launch_batch_kernel_t(const BatchArgs &B, const BatchConfig &c, cuda
         if (c.ku == 4) k_batch_persistent<D, 5, 4, FAST, BITS><<<grid, kWarps * 32, 0, s>>>(B);
         else k_batch_persistent<D, 5, 8, FAST, BITS><<<grid, kWarps * 32, 0, s>>>(B);
     } else {
-        const unsigned grid = ceil_div(B.n_segs, kWarps);
-        if (c.ku == 4) launch_batch_epoch(k_batch_epoch<D, 5, 4, FAST, BITS>, grid, B, epoch, s);
-        else launch_batch_epoch(k_batch_epoch<D, 5, 8, FAST, BITS>, grid, B, epoch, s);
+        if (c.ku == 4) launch_batch_epoch<D, 5, 4, FAST, BITS>(B, epoch, s);
+        else launch_batch_epoch<D, 5, 8, FAST, BITS>(B, epoch, s);
     }
     check_launch("k_batch");
 }
@@ -225,10 +225,9 @@ inline void launch_batch_kernel_nr0(const BatchArgs &B, const BatchConfig &c, cu
         else if (c.ku == 4) k_batch_persistent<D, 0, 4><<<grid, kWarps * 32, 0, s>>>(B);
         else k_batch_persistent<D, 0, 8><<<grid, kWarps * 32, 0, s>>>(B);
     } else {
-        const unsigned grid = ceil_div(B.n_segs, kWarps);
-        if (bits) launch_batch_epoch(k_batch_epoch<D, 0, 8, false, true>, grid, B, epoch, s);
-        else if (c.ku == 4) launch_batch_epoch(k_batch_epoch<D, 0, 4>, grid, B, epoch, s);
-        else launch_batch_epoch(k_batch_epoch<D, 0, 8>, grid, B, epoch, s);
+        if (bits) launch_batch_epoch<D, 0, 8, false, true>(B, epoch, s);
+        else if (c.ku == 4) launch_batch_epoch<D, 0, 4, false, false>(B, epoch, s);
+        else launch_batch_epoch<D, 0, 8, false, false>(B, epoch, s);
     }
     check_launch("k_batch");
 }
