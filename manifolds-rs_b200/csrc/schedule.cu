@@ -171,6 +171,35 @@ __global__ void __launch_bounds__(128) k_sched_bits(const float2 *__restrict__ s
     }
 }
 
+// The same for few words: a warp per word, a lane per entry. A thread per word
+// walks 32 dependent cursors through every epoch, 58 us for 500 epochs at 10k
+// points (k = 15, 7k words: one warp and a half an SM); a ballot an epoch takes
+// 24. With many words the ballots cost half as much again in issue slots. Lane l
+// keeps the word of epoch 32 i + l and the warp stores 32 epochs at a time.
+__global__ void __launch_bounds__(128) k_sched_bits_few(const float2 *__restrict__ sched, uint64_t n_entries,
+                                                        uint64_t words, uint32_t e_begin, uint32_t n_epochs,
+                                                        uint32_t *__restrict__ bits)
+{
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (w >= words) return;  // warp-uniform
+    const uint64_t p = w * 32 + lane;
+    const float per = p < n_entries ? sched[p].y : 0.0f;
+    float cur = p < n_entries ? per : __int_as_float(0x7f800000);  // reset: cursor = period
+    for (uint32_t e0 = 0; e0 < n_epochs; e0 += 32) {
+        uint32_t mine = 0;
+#pragma unroll 8
+        for (uint32_t l = 0; l < 32; l++) {  // (epochs past the last are walked and not stored)
+            const bool a = cur <= (float)(e0 + l);
+            const uint32_t word = __ballot_sync(0xFFFFFFFFu, a);
+            if (a) cur = cur + per;
+            if (l == lane) mine = word;
+        }
+        const uint32_t e = e0 + lane;
+        if (e >= e_begin && e < n_epochs) bits[(size_t)e * words + w] = mine;
+    }
+}
+
 // Cursors after `epochs` epochs of the schedule from the reset state.
 __global__ void k_sched_materialise(float2 *__restrict__ sched, uint64_t n_entries, uint32_t epochs)
 {
@@ -346,7 +375,11 @@ void launch_schedule_bits(const float2 *sched, uint64_t n_entries, uint32_t n_ep
 {
     const uint64_t words = (n_entries + 31) / 32;
     if (!words || e_begin >= n_epochs) return;
-    k_sched_bits<<<ceil_div(words, 128), 128, 0, s>>>(sched, n_entries, words, e_begin, n_epochs, bits);
+    // up to about three warps of words for every scheduler of the device
+    if (words <= 12u * 148u * 16u)
+        k_sched_bits_few<<<ceil_div(words * 32, 128), 128, 0, s>>>(sched, n_entries, words, e_begin, n_epochs, bits);
+    else
+        k_sched_bits<<<ceil_div(words, 128), 128, 0, s>>>(sched, n_entries, words, e_begin, n_epochs, bits);
     check_launch("k_sched_bits");
 }
 
