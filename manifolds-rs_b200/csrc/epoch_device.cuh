@@ -90,7 +90,7 @@ __device__ __forceinline__ bool checked_ok(bool ok, uint32_t *err)
 // segment's row starts overlap. (Triggered before the wait, the blocks of
 // several epochs pile up and the last of them are packed onto the few SMs with
 // room: 14 -> 24 us an epoch at 50k points.) Both are no-ops in a kernel launched
-// without the attribute (launch_after). What the previous kernel writes is
+// without the launch attribute. What the previous kernel writes is
 // written while this one may already run, so it is never read through the
 // non-coherent path or kept in L1 (COH below).
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

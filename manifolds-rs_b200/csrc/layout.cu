@@ -29,7 +29,7 @@
 // With the schedule precomputed (schedule.cu) the kernel either scans the
 // epoch's active-entry bitmask in place of the (cursor, period) pairs (BITS),
 // or reads the epoch's active-entry records without any scan (LIST). On
-// small problems both give each segment a whole block (k_epoch_split_bits,
+// small and mid-sized problems both give each segment a whole block (k_epoch_split_bits,
 // k_epoch_split). All pick the same entries in the same order and form the
 // same batches, so their results are bit-identical.
 //

@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(128) k_sched_bits(const float2 *__restrict__ s
 
 // The same for few words: a warp per word, a lane per entry. A thread per word
 // walks 32 dependent cursors through every epoch, 58 us for 500 epochs at 10k
-// points (k = 15, 7k words: one warp and a half an SM); a ballot an epoch takes
-// 24. With many words the ballots cost half as much again in issue slots. Lane l
+// points (k = 15, 7k words: one warp and a half an SM); one ballot an epoch
+// brings it to 24 us. With many words the ballots cost half as much again in issue slots. Lane l
 // keeps the word of epoch 32 i + l and the warp stores 32 epochs at a time.
 __global__ void __launch_bounds__(128) k_sched_bits_few(const float2 *__restrict__ sched, uint64_t n_entries,
                                                         uint64_t words, uint32_t e_begin, uint32_t n_epochs,
@@ -375,7 +375,9 @@ void launch_schedule_bits(const float2 *sched, uint64_t n_entries, uint32_t n_ep
 {
     const uint64_t words = (n_entries + 31) / 32;
     if (!words || e_begin >= n_epochs) return;
-    // up to about three warps of words for every scheduler of the device
+    // Twelve warps a scheduler: up to here (28k words, 40k points at k = 15) a
+    // thread per word leaves most schedulers a single warp or none; beyond, it
+    // has warps enough and the ballots' issue slots are what counts.
     if (words <= 12u * 148u * 16u)
         k_sched_bits_few<<<ceil_div(words * 32, 128), 128, 0, s>>>(sched, n_entries, words, e_begin, n_epochs, bits);
     else
