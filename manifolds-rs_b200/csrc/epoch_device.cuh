@@ -90,9 +90,12 @@ __device__ __forceinline__ bool checked_ok(bool ok, uint32_t *err)
 // segment's row starts overlap. (Triggered before the wait, the blocks of
 // several epochs pile up and the last of them are packed onto the few SMs with
 // room: 14 -> 24 us an epoch at 50k points.) Both are no-ops in a kernel launched
-// without the launch attribute. What the previous kernel writes is
-// written while this one may already run, so it is never read through the
-// non-coherent path or kept in L1 (COH below).
+// without the launch attribute. Ahead of its own grid_wait a warp reads nothing
+// but what is older than the stream's previous kernel: the row starts, and
+// arguments. That kernel need not be an epoch's -- the first epoch after a
+// schedule's build follows the one that writes the bitmasks -- and what it
+// writes is written while this one may already run, so it is never read through
+// the non-coherent path, and the embedding never kept in L1 (COH below).
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -107,6 +110,15 @@ __device__ __forceinline__ uint64_t l2_keep_policy()
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
     return pol;
+}
+
+// A bit word the previous kernel may have written (after grid_wait): a coherent
+// load.
+__device__ __forceinline__ uint32_t load_bits(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
 // How embedding buffers, moments and cursors are read; they change roles every
@@ -605,7 +617,7 @@ __device__ __forceinline__ void epoch_segment(const EpochArgs &A, WarpSmem<D, KU
             uint32_t m = 0;
             if (wb < seg_end) {
                 // the piece lies inside one word: wb is a multiple of BP
-                const uint32_t word = __ldg(A.bits + (wb >> 5));
+                const uint32_t word = COH == kDependent ? load_bits(A.bits + (wb >> 5)) : __ldg(A.bits + (wb >> 5));
                 m = BP == 32 ? word : (word >> ((uint32_t)wb & 31u)) & ((1u << (BP & 31)) - 1u);
                 if (wb < seg_beg) m &= ~0u << (seg_beg - (uint32_t)wb);
                 if (seg_end - wb < (uint32_t)BP) m &= (1u << (uint32_t)(seg_end - wb)) - 1u;
@@ -827,10 +839,11 @@ __device__ __forceinline__ void epoch_segment_split_bits(const EpochArgs &A, War
     const bool valid = node < A.n;
     float ys[D];
     if (warp == 0) load_segment<D, DENS, kDependent>(A, S, node0, lane, ys);
+    else grid_wait();  // the words may be the previous kernel's
     // masked words and their popcounts; exclusive prefix by warp 0
     for (uint32_t t = threadIdx.x; t < nw; t += blockDim.x) {
         const uint32_t wi = w0 + t;
-        uint32_t m = __ldg(A.bits + wi);
+        uint32_t m = load_bits(A.bits + wi);
         if (wi * 32u < sbeg) m &= ~0u << (sbeg - wi * 32u);
         if (wi * 32u + 32u > send) m &= (send - wi * 32u >= 32u) ? ~0u : ((1u << (send - wi * 32u)) - 1u);
         wm[t] = m;
