@@ -151,7 +151,9 @@ __global__ void k_filter_norms(const float *__restrict__ x, uint32_t n, uint32_t
                                uint32_t terms, float *__restrict__ norm, float *__restrict__ rho,
                                uint32_t *__restrict__ bad)
 {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    // (64 bits: 32 threads a row pass 2^32 from 2^27 rows on)
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t row = (uint32_t)(t >> 5), lane = threadIdx.x & 31;
     if (row >= n) return;
     double acc = 0.0;
     float second = 0.0f, rest = 0.0f;
