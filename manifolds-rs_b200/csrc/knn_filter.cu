@@ -426,15 +426,14 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
                     bulk_load(sb + (size_t)st * kBBytes, gb + (size_t)c * kBBytes, kBBytes, &full[st]);
                 }
             }
-            // what is in flight ends before the block does: the last stages'
-            // releases by the MMAs, or, when a wait gave up, the copies
+            // what is in flight ends before the block does: the copies of the
+            // last stages (the MMAs are warp 17's to wait for)
+            for (uint32_t b = it > R ? it - R : 0; b < it; b++) {
+                uint32_t none = 0;
+                bar_wait(&full[b % R], (b / R) & 1, &none);
+            }
             uint32_t none = 0;
             bar_wait(&afull, 0, &none);
-            for (uint32_t b = it > R ? it - R : 0; b < it; b++) {
-                none = 0;
-                if (ok) ok = bar_wait(&empty[b % R], (b / R) & 1, stop);
-                else bar_wait(&full[b % R], (b / R) & 1, &none);
-            }
         }
         __syncwarp();
     } else if (warp == 17) {
@@ -478,11 +477,11 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
             st0 = st;
             ph0 = ph;
         }
-        if (!ok) {  // what was issued ends before TMEM is given back
-            mma_commit(&done);
-            uint32_t none = 0;
-            bar_wait(&done, 0, &none);
-        }
+        // what was issued ends before TMEM and the staged operands are given
+        // back, whoever gave up and when
+        mma_commit(&done);
+        uint32_t none = 0;
+        bar_wait(&done, 0, &none);
     } else {
         // columns 128 half .. of accumulator b, rows 32 quarter ..
         const uint32_t b = warp >> 3, half = (warp >> 2) & 1, quarter = warp & 3;
