@@ -964,7 +964,8 @@ __global__ void __launch_bounds__(kRefineWarps * 32)
 template <int MB, int PASS, int STEPS = 0>
 void launch_filter(const FilterArgs &P, uint32_t blocks, size_t smem, cudaStream_t s)
 {
-    check_cuda(cudaFuncSetAttribute(k_filter<MB, PASS, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    // the most of any call: the attribute is the function's, shared by all threads
+    check_cuda(cudaFuncSetAttribute(k_filter<MB, PASS, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax),
                "filter shared memory");
     k_filter<MB, PASS, STEPS><<<dim3(blocks, P.slices), kFilterThreads, smem, s>>>(P);
     check_launch("k_filter");

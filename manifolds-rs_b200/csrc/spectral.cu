@@ -822,8 +822,11 @@ void batched_component_raw(uint32_t n, const DevBuf<uint64_t> &ptr, const DevBuf
     std::vector<uint32_t> found(S);
     constexpr uint32_t kTridiagRows = 110;
     if (S > 1 && it_max <= kTridiagRows) {
-        const size_t smem = 2 * sizeof(double) * it_max * (it_max | 1u);
-        check_cuda(cudaFuncSetAttribute(k_seg_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        auto smem_of = [](uint32_t r) { return 2 * sizeof(double) * r * (r | 1u); };
+        const size_t smem = smem_of(it_max);
+        // the most of any call: the attribute is the function's, shared by all threads
+        check_cuda(cudaFuncSetAttribute(k_seg_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem_of(kTridiagRows)),
                    "tridiagonal shared memory");
         k_seg_tridiag<<<S, 128, smem, s>>>(ab.p, S, it_max, kk, iters.p, c.p, dfound.p);
         check_launch("k_seg_tridiag");
