@@ -48,7 +48,9 @@ struct umapcu_state {
     ScheduleLists lists;
     ScheduleBits bits;  // the bitmask form, used when there are no lists
     DevBuf<uint32_t> err;  // checked builds: a kernel's report of a bad index
-    // layout_resident.cu: status and the epochs' counters, their scalars, the rows
+    // layout_resident.cu (one-shot layouts it takes): status and the epochs'
+    // counters, their scalars, the rows
+    bool resident = false;
     DevBuf<uint32_t> meet;
     DevBuf<float4> scal;
     DevBuf<uint4> ring;
@@ -218,8 +220,7 @@ bool run_epochs(umapcu_state *st, uint32_t first, uint32_t last, uint32_t optimi
 {
     constexpr uint32_t kSpan = 4;
     bool used = false;
-    resident = resident && st->bits_ok && !st->lists_ok && last <= st->bits.n_epochs && !st->precise_pow &&
-               st->sampler == UMAPCU_NEG_REF_HASH && st->p.neg_sample_rate == 5 && resident_takes(st->n, st->n_dim);
+    resident = resident && st->resident && st->bits_ok && !st->lists_ok && last <= st->bits.n_epochs && !st->precise_pow;
     for (uint32_t e = first; e < last;) {
         uint32_t end = e;
         while (end < last && !(st->dens && dens_active(st->lambda, st->frac, end, st->p.n_epochs))) end++;
@@ -227,10 +228,6 @@ bool run_epochs(umapcu_state *st, uint32_t first, uint32_t last, uint32_t optimi
             std::vector<float4> sc(end - e);
             for (uint32_t i = 0; i < sc.size(); i++) epoch_scalars(st->p, e + i, &sc[i].x, &sc[i].y, &sc[i].z);
             cudaStream_t s = st->stream.s;
-            if (!st->meet.p) {
-                st->meet.alloc((size_t)st->p.n_epochs + 1, s);
-                check_cuda(cudaMemsetAsync(st->meet.p, 0, sizeof(uint32_t), s), "memset status");
-            }
             st->scal.alloc(sc.size(), s);
             h2d(st->scal.p, sc.data(), sc.size(), s);
             if (!st->ring.p) st->ring.alloc(resident_ring_bytes(st->n) / sizeof(uint4), s);
@@ -363,7 +360,18 @@ umapcu_status create_state(const float *embd, uint32_t n, uint32_t n_dim, const 
         st->stats.alloc(8, s);
         check_cuda(cudaMemsetAsync(st->stats.p, 0, 8 * sizeof(float), s), "memset stats");
     }
+    // Whether all epochs can run in one launch, read back before the first of
+    // them: what follows a launch that did nothing would run on unset positions.
+    uint32_t too_long = 0;
+    if (!lists && st->bits_ok && sampler == UMAPCU_NEG_REF_HASH && params->neg_sample_rate == 5 && resident_takes(n, n_dim)) {
+        st->resident = true;
+        st->meet.alloc((size_t)params->n_epochs + 1, s);
+        check_cuda(cudaMemsetAsync(st->meet.p, 0, sizeof(uint32_t), s), "memset status");
+        launch_resident_fits(st->csr.offsets.p, n, st->meet.p, s);
+        d2h(&too_long, st->meet.p, 1, s);
+    }
     sync(s);
+    if (too_long) st->resident = false;
     T.mark("state upload", s);
     out = std::move(st);
     return UMAPCU_OK;
@@ -848,6 +856,15 @@ umapcu_status umapcu_optimise_embedding(float *embd, uint32_t n, uint32_t n_dim,
         const uint64_t nt = (uint64_t)n * n_dim;
         PhaseTimer T;
         NvtxRange r("umapcu epochs");
+        // a launch of many epochs whose blocks gave up waiting for one another
+        auto gave_up = [&]() {
+            uint32_t status = 0;
+            d2h(&status, st->meet.p, 1, st->stream.s);
+            sync(st->stream.s);
+            return status != 0;
+        };
+        uint32_t printed = 0;  // epochs up to here have their line
+        // false: the epochs were not run to their end
         auto run_all = [&](bool resident) {
             bool used = false;
             for (uint32_t e = 0; e < params->n_epochs;) {
@@ -856,6 +873,7 @@ umapcu_status umapcu_optimise_embedding(float *embd, uint32_t n, uint32_t n_dim,
                 used = run_epochs(st.get(), e, log, optimiser, resident) || used;
                 e = log;
                 if (e == params->n_epochs) break;
+                if (used && gave_up()) return false;
                 DevBuf<float> g(nt, st->stream.s);
                 run_epoch(st.get(), e, optimiser, nullptr, g.p, nullptr);
                 std::vector<float> hg(nt);
@@ -863,25 +881,21 @@ umapcu_status umapcu_optimise_embedding(float *embd, uint32_t n, uint32_t n_dim,
                 sync(st->stream.s);
                 double ss = 0.0;
                 for (float x : hg) ss += (double)x * x;
-                printf(" Epoch %u / %u: grad norm %.2f\n", e + 1, params->n_epochs, sqrt(ss));
                 e++;
+                if (e > printed) printf(" Epoch %u / %u: grad norm %.2f\n", e, params->n_epochs, sqrt(ss));
+                printed = std::max(printed, e);
             }
-            return used;
+            return !used || !gave_up();
         };
-        if (run_all(true)) {
-            uint32_t status = 0;
-            d2h(&status, st->meet.p, 1, st->stream.s);
-            sync(st->stream.s);
-            if (status) {  // a segment too long, or a wait that gave up: once more, a launch per epoch
-                cudaStream_t s = st->stream.s;
-                st->cur = 0;
-                h2d(st->y[0].p, embd, nt, s);
-                check_cuda(cudaMemsetAsync(st->m.p, 0, nt * sizeof(float), s), "memset m");
-                check_cuda(cudaMemsetAsync(st->v.p, 0, nt * sizeof(float), s), "memset v");
-                st->sched_epoch = 0;
-                st->sched_continuous = true;
-                run_all(false);
-            }
+        if (!run_all(true)) {  // once more, a launch per epoch
+            cudaStream_t s = st->stream.s;
+            st->cur = 0;
+            h2d(st->y[0].p, embd, nt, s);
+            check_cuda(cudaMemsetAsync(st->m.p, 0, nt * sizeof(float), s), "memset m");
+            check_cuda(cudaMemsetAsync(st->v.p, 0, nt * sizeof(float), s), "memset v");
+            st->sched_epoch = 0;
+            st->sched_continuous = true;
+            run_all(false);
         }
         T.mark("epochs", st->stream.s);
         d2h(embd, st->y[st->cur].p, nt, st->stream.s);

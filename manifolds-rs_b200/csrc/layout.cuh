@@ -68,14 +68,17 @@ void launch_epoch(const EpochArgs &A, uint32_t n_dim, bool dens, cudaStream_t s)
 // segments (four blocks on each of 148 SMs).
 constexpr uint32_t kResidentSegments = 148 * 4;
 bool resident_takes(uint32_t n, uint32_t n_dim);
+// Sets *status (device) to UMAPCU_CAPACITY when a segment of the graph is too
+// long for a block: launch_layout_resident must then not be called.
+void launch_resident_fits(const uint32_t *offsets, uint32_t n, uint32_t *status, cudaStream_t s);
 // Epochs [first, first + count) of the fast configuration (hash sampler, five
 // negatives, no density term, approximate powers) from A.y_cur, the last
 // written to A.y_cur (count even) or A.y_next (odd). A.bits is the bitmask of
 // epoch 0, `words` its words per epoch, scal the epochs' {fused, epsc, lr, 0},
 // ring scratch of resident_ring_bytes, counter scratch of count words, status a
-// zeroed word that is set when the epochs were not run to their end:
-// UMAPCU_TIMEOUT, a wait between blocks gave up; UMAPCU_CAPACITY, a segment is
-// too long. false: the device cannot hold all blocks at once, nothing was run.
+// zeroed word that is set to UMAPCU_TIMEOUT when a wait between blocks gave up
+// and the epochs were not run to their end. false: the device cannot hold all
+// blocks at once, nothing was run.
 size_t resident_ring_bytes(uint32_t n);
 bool launch_layout_resident(const EpochArgs &A, uint32_t n_dim, const float4 *scal, uint32_t first, uint32_t count,
                             uint64_t words, uint4 *ring, uint32_t *counter, uint32_t *status, cudaStream_t s);

@@ -113,7 +113,7 @@ __device__ __forceinline__ void gather(const uint4 *slot, uint32_t tag, uint32_t
 }
 
 // *status set to UMAPCU_CAPACITY when a segment has more bit words than a
-// block holds: the resident kernel then does nothing.
+// block holds.
 __global__ void k_resident_fits(const uint32_t *__restrict__ offsets, uint32_t n, uint32_t *__restrict__ status)
 {
     const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) * 32u;
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * (NG * G + 1), MIN_BLOCKS)
     __shared__ uint32_t words_of[NG][kSplitWords], before[NG][G][kSplitWords], active_of[NG];
     __shared__ uint2 entries[kEntries];
     __shared__ volatile bool stop;
-    if (*status) return;  // grid-uniform: k_resident_fits has set it, or an earlier span gave up
+    if (*status) return;  // an earlier span gave up
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t node0 = blockIdx.x * 32u, node = node0 + lane;
     const uint32_t n = A.n;
@@ -330,8 +330,6 @@ bool try_launch(const EpochArgs &A, const float4 *scal, uint32_t first, uint32_t
     int per_sm = 0;
     check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0), "occupancy");
     if ((uint64_t)per_sm * device_sm_count() < nseg) return false;
-    k_resident_fits<<<ceil_div(nseg, 256), 256, 0, s>>>(A.offsets, A.n, status);
-    check_launch("k_resident_fits");
     check_cuda(cudaMemsetAsync(counter, 0, sizeof(uint32_t) * count, s), "memset counter");
     check_cuda(cudaMemsetAsync(ring, 0, resident_ring_bytes(A.n), s), "memset ring");  // no row carries a tag yet
     EpochArgs a = A;
@@ -369,6 +367,12 @@ size_t resident_ring_bytes(uint32_t n) { return (size_t)kRing * n * sizeof(uint4
 bool resident_takes(uint32_t n, uint32_t n_dim)
 {
     return (n_dim == 2 || n_dim == 3) && ceil_div(n, 32) <= kResidentSegments;
+}
+
+void launch_resident_fits(const uint32_t *offsets, uint32_t n, uint32_t *status, cudaStream_t s)
+{
+    k_resident_fits<<<ceil_div(ceil_div(n, 32), 256), 256, 0, s>>>(offsets, n, status);
+    check_launch("k_resident_fits");
 }
 
 bool launch_layout_resident(const EpochArgs &A, uint32_t n_dim, const float4 *scal, uint32_t first, uint32_t count,
