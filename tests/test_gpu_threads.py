@@ -37,17 +37,18 @@ def test_searches_and_spectral_starts_of_different_widths():
               for x, k in ((data[0], 10), (data[1], 31))]
     calls += [lambda d=d: umapcu.spectral_layout(graph, d, 1) for d in (2, 3, 10)]
     want = [f() for f in calls]
+    repeats = [120, 120, 60, 60, 60, 60, 10, 10, 10]
     wrong = []
 
     def work(i):
         try:
-            for _ in range(25):
+            for _ in range(repeats[i]):
                 if not np.array_equal(calls[i](), want[i]):
                     wrong.append(i)
         except Exception as e:  # noqa: BLE001
             wrong.append((i, repr(e)))
 
-    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    threads = [threading.Thread(target=work, args=(i,)) for i in [0, 1, 0, 1] + list(range(len(calls)))]
     for t in threads:
         t.start()
     for t in threads:
