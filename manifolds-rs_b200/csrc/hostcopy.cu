@@ -13,7 +13,11 @@
 //
 // The block is one per process, page-locked for every device, allocated at the
 // first large copy and given back by umapcu_release_cached. A copy that finds
-// it taken by another thread's goes through the runtime as before.
+// it taken by another thread's goes through the runtime as before, and so does
+// one whose context is not its device's primary one: the helping threads, and
+// the block, belong to primary contexts.
+#include <cuda.h>
+
 #include <atomic>
 #include <mutex>
 #include <thread>
@@ -40,6 +44,37 @@ unsigned copy_threads()
 {
     static const unsigned n = std::min(kMaxThreads, std::thread::hardware_concurrency() / 2);
     return n;
+}
+
+// Whether the calling thread's context is the primary one of device dev.
+bool primary_context(int dev)
+{
+    struct Calls {
+        decltype(&cuCtxGetCurrent) current = nullptr;
+        decltype(&cuDevicePrimaryCtxRetain) retain = nullptr;
+        decltype(&cuDevicePrimaryCtxRelease) release = nullptr;
+        Calls()
+        {
+            auto get = [](const char *name, auto &f) {
+                cudaDriverEntryPointQueryResult found;
+                void *p = nullptr;
+                if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &found) == cudaSuccess &&
+                    found == cudaDriverEntryPointSuccess)
+                    f = reinterpret_cast<std::remove_reference_t<decltype(f)>>(p);
+                else cudaGetLastError();
+            };
+            get("cuCtxGetCurrent", current);
+            get("cuDevicePrimaryCtxRetain", retain);
+            get("cuDevicePrimaryCtxRelease", release);
+        }
+    };
+    static const Calls f;
+    if (!f.current || !f.retain || !f.release) return false;
+    CUcontext mine = nullptr, primary = nullptr;
+    // (a runtime device is the driver's of the same number)
+    if (f.current(&mine) != CUDA_SUCCESS || !mine || f.retain(&primary, dev) != CUDA_SUCCESS) return false;
+    f.release(dev);
+    return mine == primary;
 }
 
 struct Block {
@@ -140,6 +175,7 @@ bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaS
     if (at.type != cudaMemoryTypeUnregistered) return false;  // page-locked already
     int dev = 0;
     check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (!primary_context(dev)) return false;
     Block block;
     if (!block.p) return false;
     if (!to_device) sync(s);  // not by the copying threads, which would spin
@@ -147,7 +183,7 @@ bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaS
     std::atomic<size_t> next{0};
     cudaError_t err[kMaxThreads] = {};
     auto work = [&](unsigned t) {
-        err[t] = cudaSetDevice(dev);
+        if (t) err[t] = cudaSetDevice(dev);  // the calling thread's context is as it should be
         if (err[t] == cudaSuccess)
             err[t] = move_chunks(static_cast<uint8_t *>(dst), static_cast<const uint8_t *>(src), bytes, to_device,
                                  block.p + 2 * kChunk * t, next, s);
