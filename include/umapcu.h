@@ -435,9 +435,10 @@ umapcu_status umapcu_state_schedule_form(const umapcu_state *st, uint32_t *form)
 
 /* ---------------------------------------------------- memory hygiene
  * (no counterpart in the reference, whose UmapGpuState holds device memory
- * for one call only, umap_optimiser_gpu.rs:278-348). The library keeps two
+ * for one call only, umap_optimiser_gpu.rs:278-348). The library keeps three
  * things between calls: the one-shot call's schedule-bitmask block (one per
- * device, up to 1 bit per CSR entry and epoch) and, in each device's default
+ * device, up to 1 bit per CSR entry and epoch), a page-locked block (16 MB for
+ * the process) that large copies go through and, in each device's default
  * stream-ordered memory pool (a process-wide object), the blocks its calls
  * freed -- it raises that pool's release threshold, which otherwise returns
  * freed memory to the driver at every synchronisation. */

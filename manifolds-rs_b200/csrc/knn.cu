@@ -631,6 +631,7 @@ umapcu_status umapcu_knn_exact_dev(const float *d_x, uint32_t n, uint32_t dim, c
     return guard_k([&]() -> umapcu_status {
         if (n == 0) return UMAPCU_NO_DATA;
         if (!d_x || !d_idx || !d_dist || n >= (1u << 31)) return UMAPCU_BAD_ARG;
+        keep_pool_memory();  // the filter's scratch: mapping 380 MB for 1M x 50 anew takes 4 ms
         knn_dev(d_x, n, dim, d_queries, n_queries, k, metric, d_idx, d_dist, (cudaStream_t)stream);
         return UMAPCU_OK;
     });

@@ -1054,19 +1054,29 @@ uint32_t rank_stages(uint32_t chunks, uint32_t k)
 
 }  // namespace
 
-// The filter's fixed cost (packing, eight launches) is some tens of
-// microseconds, so it takes searches of at least kFilterPairs pairs; below
-// kFilterPoints points the sample is too small for its groups, and beyond 191
-// dims the operands no longer fit beside the ring. Whole calls, k = 15, us,
-// k_knn_tile -> filter: 2048 points x 2 / 50 / 190 dims 472 -> 306, 514 -> 354,
-// 628 -> 569; 4096 points 646 -> 338, 753 -> 435, 1120 -> 786; 6000 x 190
-// 1705 -> 929.
+// The filter prepares all points for whatever number of queries, so it takes
+// searches of at least kFilterPairs pairs whose queries are enough to pay for
+// that: (500 + 10 dim) sqrt(3 / k) up to 12 000 points, fewer beyond (a tile
+// kernel of few queries keeps its SMs busy the longer, the filter's few blocks
+// do not), but from 160 + n / 4000 on. (The preparation of n points and the
+// tile kernel's work per query are both linear in n; a longer list costs the
+// tile kernel more.) Below kFilterPoints points the sample is too small for
+// its groups, and beyond 191 dims the operands no longer fit beside the ring.
+// us, k_knn_tile and the filter, queries chosen from n points on the device:
+//   10k x 50, k = 3     256 queries 134, 180   1000 178, 189    2000 265, 205
+//   100k x 190, k = 15  256 980, 1241          1000 2430, 1247
+//   1M x 50, k = 3      64 633, 1777           256 1689, 1751   512 3099, 1816
+// and whole calls over all points, k = 15: 2048 points x 2 / 50 / 190 dims 472,
+// 306; 514, 354; 628, 569; 4096 points 646, 338; 753, 435; 1120, 786.
 bool knn_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k)
 {
     constexpr uint32_t kFilterPoints = 2048;
     constexpr uint64_t kFilterPairs = 4u << 20;
-    return n >= kFilterPoints && (uint64_t)n * nq >= kFilterPairs && pack_of(dim).chunks <= kMaxChunks &&
-           n < (1u << 30) && k + 1 < kGroups;
+    if (n < kFilterPoints || n >= (1u << 30) || (uint64_t)n * nq < kFilterPairs || k + 1 >= kGroups) return false;
+    if (dim > 3u * kChunkK || pack_of(dim).chunks > kMaxChunks) return false;
+    const double few = (500.0 + 10.0 * dim) * std::min(1.0, std::sqrt(12000.0 / n));
+    const double least = std::sqrt(3.0 / k) * std::max(std::min(512.0, 160.0 + n / 4000.0), few);
+    return nq >= least;
 }
 
 bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaStream_t s)

@@ -27,9 +27,10 @@ def _rings(n, parts, seed):
 
 def test_searches_and_spectral_starts_of_different_widths():
     rng = np.random.default_rng(0)
-    # 30 dims: two blocks of queries a block, 50 dims: as many in more shared
-    # memory, 100 and 150: one; k = 10 and 31: tables of different length
-    data = [rng.normal(size=(3000, dim)).astype(np.float32) for dim in (30, 50, 100, 150)]
+    # 20 and 50 dims: two blocks of queries a block in 193 and 225 KB of shared
+    # memory, 100 and 150: one block in 209 and 225 KB; k = 10 and 31: tables of
+    # different length
+    data = [rng.normal(size=(3000, dim)).astype(np.float32) for dim in (20, 50, 100, 150)]
     q = rng.choice(3000, 1500, replace=False).astype(np.uint32)
     graph = _rings(60, 8, 1)
     calls = [lambda x=x: umapcu.knn_exact(x, 10)[0] for x in data]
