@@ -380,6 +380,15 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
     uint8_t *sb = sa + (size_t)MB * P.chunks * kABytes;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slice = blockIdx.y;
+    if constexpr (PASS == 2) {  // a block without a query to be listed has nothing to contract
+        const uint32_t q = blockIdx.x * MB * kBlkM + threadIdx.x;
+        const bool in = threadIdx.x < MB * kBlkM && q < P.nq;
+        if (!__syncthreads_or(in && P.least[q] < __int_as_float(0x7f800000))) {
+            constexpr uint32_t kParts = MB == 2 ? 2 : 4;  // of a slice
+            for (uint32_t p = 0; in && p < kParts; p++) P.count[(size_t)(slice * kParts + p) * P.nq + q] = 0;
+            return;
+        }
+    }
     const uint32_t sampled = (P.n_tiles + P.stride - 1) / P.stride;
     const uint32_t n_items = sampled > slice ? (sampled - slice + P.slices - 1) / P.slices : 0;
     if (threadIdx.x == 0) {
@@ -696,9 +705,14 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_filter(const FilterArgs P
 // D (1 + 4 gamma)) / 2 less the bound. Cosine: scores are the dot products of
 // unit rows, E = 2.1 kappa, the chain's rounding dim 2^-24 on both sides and
 // that of 1 - dot.
+// A query with every group's maximum at or above that least score (some 300
+// points of the sample are, in 64 groups) has more candidates than its lists
+// hold or pay for: give_up (knn_filter) sends it on without listing any. The
+// points of tight clusters far apart or of equal rows all are such: 200k x 30
+// dims 163.6 -> 151.4 ms (151.1 by the tile kernel alone).
 __global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t parts, uint32_t nq, uint32_t k,
                                    const float *__restrict__ norm, const uint32_t *__restrict__ qidx, uint32_t q0,
-                                   uint32_t dim, bool euc, const float *__restrict__ rho, uint32_t steps,
+                                   uint32_t dim, bool euc, const float *__restrict__ rho, uint32_t steps, bool give_up,
                                    float *__restrict__ least)
 {
     const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -723,7 +737,6 @@ __global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t part
             else o1 = 0;
         }
     }
-    if (lane != 0) return;
     const double kappa = filter_kappa(rho, steps);
     const double s = (double)__uint_as_float((top & 0x80000000u) ? top ^ 0x80000000u : ~top);
     double g;
@@ -737,7 +750,18 @@ __global__ void k_filter_threshold(const float *__restrict__ gmax, uint32_t part
     } else {
         g = s - 2.0 * 2.1 * kappa - (2.0 * dim + 16.0) * 0x1p-24 - 0x1p-22;
     }
-    least[q] = __double2float_rd(g);
+    const float l = __double2float_rd(g);
+    const bool all = __all_sync(kFull, v0 >= l && v1 >= l);
+    if (lane == 0) least[q] = give_up && all ? __int_as_float(0x7f800000) : l;
+}
+
+// The candidates listed for query q, all parts together.
+__device__ __forceinline__ uint32_t listed(const uint32_t *__restrict__ count, uint32_t parts, uint32_t nq, uint32_t q,
+                                           uint32_t lane)
+{
+    uint32_t c = 0;
+    for (uint32_t p = lane; p < parts; p += 32) c += min(count[(size_t)p * nq + q], 1u << 20);
+    return __reduce_add_sync(kFull, c);
 }
 
 __device__ __forceinline__ bool better(float d, uint32_t i, float td, uint32_t ti)
@@ -786,8 +810,10 @@ __device__ __forceinline__ float chain_distance(const float *__restrict__ x, uin
 
 // The exact second look, a warp per query: 32 candidates at a time, their
 // chain distances, and insertion into the warp's sorted list (lane l holds
-// entry l). A query whose lists overflowed, or any query when *bad, goes to
-// left.
+// entry l). A query whose lists overflowed or hold more than a quarter of the
+// points (row by row that costs more than the tile kernel's pass over all;
+// metrics of 3000 equal rows, whole call: 1.39 -> 0.71 ms, 0.64 by the tile
+// kernel alone), or any query when *bad, goes to left.
 constexpr int kRefineWarps = 4;
 template <bool EUC>
 __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__restrict__ x, uint32_t n, uint32_t dim, uint32_t k,
@@ -804,7 +830,7 @@ __global__ void __launch_bounds__(kRefineWarps * 32) k_refine(const float *__res
     const uint32_t q = blockIdx.x * kRefineWarps + warp;
     if (q >= nq) return;  // warp-uniform
     const uint32_t self = qidx ? qidx[q0 + q] : q0 + q;
-    bool over = *bad != 0;
+    bool over = *bad != 0 || (n / 4 < parts * cap && listed(count, parts, nq, q, lane) > n / 4);
     float ld = __int_as_float(0x7f800000);
     uint32_t li = ~0u;
     for (uint32_t p = 0; !over && p < parts; p++) {
@@ -920,7 +946,7 @@ __global__ void __launch_bounds__(kRefineWarps * 32)
     const uint32_t q = blockIdx.x * kRefineWarps + warp;
     if (q >= nq) return;  // warp-uniform
     const uint32_t self = qidx ? qidx[q0 + q] : q0 + q;
-    bool over = *bad != 0;
+    bool over = *bad != 0 || (n / 4 < parts * cap && listed(count, parts, nq, q, lane) > n / 4);
     const size_t at = (size_t)(q0 + q) * k;
     uint32_t c_m = 0, g = 0, tj = 0;
     float td = 0.0f;
@@ -1091,6 +1117,7 @@ bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaSt
     // points of all reach it
     const double r = -(double)kGroups * std::log(1.0 - (double)(A.k + 1) / kGroups);
     const uint32_t stride = std::max(1u, std::min((uint32_t)(kHitTarget / r), n_tiles / 4));
+    const bool give_up = 320 * stride >= std::min(A.n / 4, kListCap);
     // queries in batches of at most two waves of blocks (four with one block of
     // queries each): bounds the scratch
     const uint32_t rows = MB * kBlkM, batch = std::min<uint32_t>(ceil_div(A.nq, rows), (MB == 2 ? 2 : 4) * sms) * rows;
@@ -1131,7 +1158,7 @@ bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaSt
         if (MB == 2) launch_filter<2, 1>(P, blocks, smem, s);
         else launch_filter<1, 1>(P, blocks, smem, s);
         k_filter_threshold<<<ceil_div((uint64_t)nq * 32, 256), 256, 0, s>>>(
-            gmax.p, P.slices * per, nq, A.k, K.norm.p, A.qidx, q0, A.dim, A.euc, K.rho.p, pk.steps, least.p);
+            gmax.p, P.slices * per, nq, A.k, K.norm.p, A.qidx, q0, A.dim, A.euc, K.rho.p, pk.steps, give_up, least.p);
         check_launch("k_filter_threshold");
         P.stride = 1;
         P.slices = slices_of(blocks, n_tiles);

@@ -67,3 +67,38 @@ def test_ranks_of_several_batches_of_queries():
     sub = rng.choice(n, 60, replace=False)
     got = umapcu.embedding_quality(X, Y, None, k, queries=sub)["trust"]
     assert got == O.trustworthiness(X, Y, k, queries=sub.astype(np.uint32))
+
+
+# queries the filter cannot settle (their equal rows overflow a candidate list),
+# among others it settles: one, just below, at and above a group of 64, and
+# nearly all; few of them split the points, many do not
+@pytest.mark.parametrize("metric,members", [("euclidean", (1, 63, 64, 65, 390)), ("cosine", (2, 300))])
+def test_queries_left_by_the_filter(metric, members):
+    n, dim, k = 50_000, 20, 3
+    rng = np.random.default_rng(8)
+    X = rng.normal(size=(n, dim)).astype(np.float32)
+    X[20_000:20_600] = X[20_000]  # more equal rows in a tile than a part's list holds
+    others = np.concatenate([np.arange(0, 20_000, 37), np.arange(21_000, n, 37)])
+    for m in members:
+        inside = 20_000 + rng.permutation(600)[:m]
+        q = rng.permutation(np.concatenate([inside, others[: 400 - m]]))
+        gi, gd = _chosen(X, q, k, metric)
+        for part in np.array_split(np.arange(q.size), 4):  # 100 queries: the tile kernel
+            ti, td = _chosen(X, q[part], k, metric)
+            assert np.array_equal(gi[part], ti) and np.array_equal(gd[part], td)
+
+
+def test_all_queries_left_by_the_filters():
+    """Tight clusters far apart: every list overflows, and all queries make more
+    groups than blocks."""
+    n, k = 40_000, 5
+    rng = np.random.default_rng(9)
+    X = (10 * rng.normal(size=(4, 8))[rng.integers(0, 4, n)] + 1e-3 * rng.normal(size=(n, 8))).astype(np.float32)
+    gi, gd = umapcu.knn_exact(X, k)
+    q = rng.permutation(n)[:200]
+    ti, td = _chosen(X, q, k, "euclidean")
+    assert np.array_equal(gi[q], ti) and np.array_equal(gd[q], td)
+    Y = X[:, :2].copy()
+    sub = rng.permutation(n)[:1000].astype(np.uint32)
+    t = [umapcu.embedding_quality(X, Y, None, k, queries=s)["trust"] for s in [sub] + list(sub.reshape(10, 100))]
+    assert abs(t[0] - np.mean(t[1:])) < 1e-13
