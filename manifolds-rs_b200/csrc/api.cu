@@ -90,7 +90,7 @@ void validate_params(const umapcu_optim_params *p, uint32_t n_dim)
     if (p->n_epochs == 0) fail(UMAPCU_BAD_ARG, "n_epochs must be positive");
 }
 
-void dens_update(umapcu_state *st)
+void dens_update(umapcu_state *st, bool dependent = false)
 {
     DensArgs D{};
     D.n = st->n;
@@ -110,7 +110,7 @@ void dens_update(umapcu_state *st)
     D.precise_pow = st->precise_pow;
     D.n_entries = 2 * st->csr.n_edges;
     D.err = st->err.p;
-    launch_dens_update(D, st->n_dim, st->stream.s);
+    launch_dens_update(D, st->n_dim, dependent, st->stream.s);
 }
 
 // Cursors in csr.sched brought up to date (after list-mode epochs).
@@ -187,7 +187,6 @@ void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint3
                uint32_t *d_act, bool skip_dens = false)
 {
     const bool dens_on = st->dens && dens_active(st->lambda, st->frac, epoch, st->p.n_epochs);
-    if (dens_on && !skip_dens) dens_update(st);
     const bool in_order = st->sched_continuous && epoch == st->sched_epoch;
     const bool use_lists = st->lists_ok && in_order && epoch < st->lists.n_epochs;
     const bool use_bits = !use_lists && st->bits_ok && in_order && epoch < st->bits.n_epochs;
@@ -208,6 +207,7 @@ void run_epoch(umapcu_state *st, uint32_t epoch, uint32_t optimiser, const uint3
     A.injected = d_inj;
     A.dbg_grad = d_grad;
     A.dbg_active = d_act;
+    if (dens_on && !skip_dens) dens_update(st, density_radii_dependent(A, st->n_dim));
     launch_epoch(A, st->n_dim, dens_on, st->stream.s);
     st->cur ^= 1;
 }

@@ -454,13 +454,81 @@ static void launch_one(void (*kernel)(Args), unsigned grid, unsigned threads, co
 // of the 148 SMs) a segment gets a whole block in every configuration.
 constexpr uint32_t kSplitSegments = 148 * 9;
 
+// Warps the device holds of the kernels with six blocks an SM.
+static uint32_t six_block_warps() { return 6u * kWarps * (uint32_t)device_sm_count(); }
+
+static bool fast_config(const EpochArgs &A)
+{
+    return !A.injected && A.sampler == UMAPCU_NEG_REF_HASH && !A.precise_pow && A.neg_rate == 5;
+}
+
 // How an epoch is launched: `warps` per segment in a block of its own, or 0 for
 // k_epoch (a warp per segment); dependent on the kernel before or after its end.
 struct EpochForm {
     int warps;
     bool dependent;
-    bool plain() const { return !warps && !dependent; }
+    bool radii_dependent;  // density epochs: the radii's kernel likewise
 };
+
+// Density epochs: radii (four segments a block), then the epoch. A grid placed
+// while the one before it drains is packed onto the SMs that are free first, and
+// by how much that costs changes from size to size: with both kernels dependent
+// epochs of 500 to 4600 segments took up to twice as long (scan, 2-D, 20k points
+// 27.6 us, dependent 36, 3-D 40 and 72; bitmasks, 8-D, 45k 103 and 162). So each
+// is dependent only where it gained at all sizes measured. us an epoch, k = 15,
+// all launched after their predecessors (eight warps with bitmasks and four with
+// lists up to 1331 segments, k_epoch beyond) -> this form; P: six_block_warps.
+//  * split epochs behind the radii, which end together: dependent, the radii not,
+//    six warps with bitmasks, three with lists: 2-D bitmasks 700 segments 26.1 ->
+//    22.7, 1407 32.4 -> 28.9, 3-D 37.1 -> 31.0, 51.1 -> 46.4, 8-D 1000 81.4 -> 76.6;
+//    lists 3-D 800 35.0 -> 32.9, 8-D 77.3 -> 75.3.
+//  * both, where few blocks find room beside any grid: lists up to 560 segments
+//    (2-D 22.7 -> 18.6; general kernels to 700; 444 above four dimensions), in one, two and four dimensions
+//    to 1000 (800: 26.3 -> 20.5; 3-D 35.0 -> 35.6); bitmasks to 500 (22.7 -> 17.1;
+//    3-D at 440 26.9 -> 30.7, four negatives 21.6 -> 27.0), scans to 444; and a warp
+//    per segment on lists to 0.53 P (1407: 31.4 -> 26.8).
+//  * the radii alone, where the epoch is k_epoch: to 0.53 P (scans 2-D 1000: 30.9
+//    -> 28.7), in one and two dimensions to 1.3 P (2344: 36.6 -> 34.6; 3-D 2813 69.6
+//    -> 88, scans 42.6 -> 45.0).
+//  * the epoch alone from P on, three warps a segment above two dimensions (3-D
+//    120k points 90.0 -> 84.1), and both from 4/3 P on, where grids run in waves
+//    (200k: 66.1 -> 62.5, 3-D 125 -> 114, 400k 115 -> 112), three warps to 2 P (1.8 P
+//    in two dimensions; bitmasks in four dimensions keep k_epoch).
+static EpochForm density_form(const EpochArgs &A, uint32_t n_dim)
+{
+    const uint32_t nseg = ceil_div(A.n, 32), P = six_block_warps();
+    const bool fast5 = fast_config(A), lists = A.rec != nullptr, bits = !lists && A.bits;
+    const bool even = n_dim <= 2 || n_dim == 4;  // (rows of one load)
+    const bool three = fast5 && (lists || (bits && n_dim != 4));
+    if (3 * nseg > 4 * P) {
+        if (three && nseg <= (n_dim <= 2 ? P / 10 * 18 : 2 * P)) return {3, true, true};
+        return {0, true, n_dim <= 4 || !bits};
+    }
+    if (nseg > P && (lists || bits)) {
+        if (three && (n_dim > 2 || 10 * nseg > 13 * P)) return {3, true, false};
+        if (fast5 && n_dim <= 2) return {0, false, true};
+        return {0, true, false};
+    }
+    if (100 * nseg > 53 * P) return {0, false, fast5 && n_dim <= 2 && (lists || bits)};
+    if (lists) {
+        if (n_dim > 4) {
+            if (nseg < kSplitSegments) return {4, true, nseg <= 444};
+            return fast5 ? EpochForm{3, true, false} : EpochForm{0, false, false};
+        }
+        if (nseg >= kSplitSegments) return {0, true, true};
+        if (nseg <= (fast5 ? 560u : 700u)) return {4, true, true};
+        return {fast5 ? 3 : 4, true, fast5 && even && nseg <= 1000};
+    }
+    if (bits) {
+        if (fast5) return even && nseg <= 500 ? EpochForm{8, true, true} : EpochForm{6, true, false};
+        if (nseg < kSplitSegments) return {8, true, false};
+        return {0, false, n_dim <= 4};
+    }
+    if (even && nseg <= 444) return {0, true, true};
+    return {0, false, !A.precise_pow && (n_dim <= 4 || nseg < kSplitSegments)};
+}
+
+bool density_radii_dependent(const EpochArgs &A, uint32_t n_dim) { return density_form(A, n_dim).radii_dependent; }
 
 // The form by the number of segments; P is how many warps of k_epoch the device
 // holds at once. us an epoch, fast configuration, k = 15, two dimensions unless
@@ -470,36 +538,57 @@ struct EpochForm {
 //    (42k: 6 10.9, 8 11.5, k_epoch 11.6; 60k: 13.1, k_epoch 13.8), in three
 //    dimensions up to half (50k: 21.9, k_epoch 23.4). Lists need no ranks and
 //    take six up to 444 segments (10k: 5.5, four 6.3) and three up to 1000 (30k:
-//    7.9, six 9.1), in three dimensions six up to half of P (50k: 20.8, k_epoch
-//    22.6). With the density term eight (bitmasks) or four (lists).
+//    7.9, six 9.1), in more dimensions six up to half of P (3-D 50k: 20.8, k_epoch
+//    22.6) but for the sizes whose blocks do not fit beside the previous grid's:
+//    three warps launched after it in three dimensions from 900 to 1331 segments
+//    (1100: 17.1, six 18.0, four 17.7) and above four up to 800 (5-D 440: 14.2, six
+//    15.5; 8-D 560: 22.0, six 27.7), then four (5-D 1100: 24.4, six 26.7), and in
+//    four dimensions from 850 four (1100: 9.1, six 10.8) and from 1150 three
+//    (1330: 10.6, six 11.5).
 //  * up to half of P: k_epoch, dependent.
 //  * between P / 2 and P a dependent grid does not fit beside the one before
 //    it, its first blocks are packed onto what is left of the SMs and the epoch
 //    takes a third longer (100k points 24.9 us, launched after 18.8); just above
 //    P the last few warps make a round of their own. Blocks of three warps a
 //    segment spread evenly: 100k 17.5, 200k 29.8 (k_epoch 31.7), 200k in three
-//    dimensions 68 (72), 200k densMAP 53 (55.6), up to 1.27 P in two dimensions
-//    (250k: 35.8, k_epoch 35.7) and 2 P in the kernels of six blocks an SM;
-//    from 0.78 P (with the density term from P / 2) to P k_epoch launched after
-//    its predecessor is as good in two dimensions (160k: 24.3, three warps
-//    25.0; 70k densMAP, k = 30: 26.4 and 27.6).
+//    dimensions 68 (72), in eight 160 (168), up to 1.27 P in two dimensions (250k:
+//    35.8, k_epoch 35.7) and 2 P in the kernels of six blocks an SM; from 0.78 P to
+//    P k_epoch launched after its predecessor is as good in two dimensions (160k:
+//    24.3, three warps 25.0). In four dimensions bitmasks keep k_epoch (180k: 31.6,
+//    three warps 35.6).
 //  * beyond: k_epoch, dependent (1M 112.7, launched after 114.5).
+// Several layouts at once on one device fill each other's gaps, and the blocks
+// of several warps a segment are then overhead: four states on threads of their
+// own, bitmasks, us an epoch each, k_epoch and this form: 60k points 7.0 and 9.3,
+// 100k 10.5 and 12.4, 200k 20.6 and 25.7 (alone 16.7 and 13.7, 19.8 and 18.6, 35.0
+// and 30.7). The forms are chosen for one layout; many go into a batch.
 template <int D, bool DENS>
-static EpochForm epoch_form(uint32_t nseg, bool lists, bool fast5)
+static EpochForm epoch_form(const EpochArgs &A)
 {
+    const uint32_t nseg = ceil_div(A.n, 32);
+    const bool lists = A.rec != nullptr, scan = !A.rec && !A.bits, fast5 = fast_config(A);
+    if (DENS) return density_form(A, D);
+    if (scan) {
+        const uint32_t P = six_block_warps();
+        return {0, 2 * nseg <= P || nseg > 2 * P};
+    }
     if (!fast5) {
-        const uint32_t P = epoch_min_blocks<D, DENS, false>() * kWarps * (uint32_t)device_sm_count();
+        const uint32_t P = six_block_warps();
         if (nseg < kSplitSegments) return {lists ? 4 : 8, true};
-        return {0, 2 * nseg <= P || nseg > P};
+        // (powf: 120k points 29.9 launched after, 31.8 dependent)
+        return {0, 2 * nseg <= P || nseg > (A.precise_pow ? P / 10 * 13 : P)};
     }
     const uint32_t P = epoch_min_blocks<D, DENS, true>() * kWarps * (uint32_t)device_sm_count();
-    if (DENS) {
-        if (nseg < kSplitSegments) return {lists ? 4 : 8, true};
-    } else if (D > 2) {
-        if (lists || nseg >= 700) {
+    if (D > 2) {
+        if (lists) {
+            if (D > 4 && nseg < kSplitSegments) return {nseg <= 800 ? 3 : 4, false};
+            if (D == 3 && nseg > 900 && nseg < kSplitSegments) return {3, false};
+            if (D == 4 && nseg > 850 && nseg < kSplitSegments) return {nseg <= 1150 ? 4 : 3, true};
             if (2 * nseg <= P) return {6, true};
         } else {
-            return {8, true};
+            if (nseg < 700) return {8, true};
+            if (2 * nseg <= P) return {6, true};
+            if (D == 4) return {0, nseg > P};
         }
     } else if (lists) {
         if (nseg <= 444) return {6, true};
@@ -509,50 +598,56 @@ static EpochForm epoch_form(uint32_t nseg, bool lists, bool fast5)
         if (3 * nseg <= P) return {6, true};
     }
     if (2 * nseg <= P) return {0, true};
-    if (D <= 2 && nseg <= P && (DENS || nseg > P / 100 * 78)) return {0, false};
-    if (nseg <= (D <= 2 && !DENS ? P / 100 * 127 : 2 * P)) return {3, true};
+    if (D <= 2 && nseg <= P && nseg > P / 100 * 78) return {0, false};
+    if (nseg <= (D <= 2 ? P / 100 * 127 : 2 * P)) return {3, true};
     return {0, true};
+}
+
+// k_epoch on the schedule the arguments carry. PLAIN: after the end of the
+// previous kernel, reading through the non-coherent path.
+template <int D, bool DENS, int NR, bool FAST, bool PLAIN>
+static void launch_warps(const EpochArgs &A, bool dependent, cudaStream_t s)
+{
+    const unsigned grid = ceil_div(ceil_div(A.n, 32), kWarps);
+    if (A.rec) launch_one(k_epoch<D, DENS, NR, FAST, true, false, PLAIN>, grid, kWarps * 32, A, dependent, s);
+    else if (A.bits) launch_one(k_epoch<D, DENS, NR, FAST, false, true, PLAIN>, grid, kWarps * 32, A, dependent, s);
+    else launch_one(k_epoch<D, DENS, NR, FAST, false, false, PLAIN>, grid, kWarps * 32, A, dependent, s);
 }
 
 template <int D, bool DENS>
 static void launch_epoch_t(const EpochArgs &A, cudaStream_t s)
 {
     const uint32_t nseg = ceil_div(A.n, 32);
-    const bool fast = !A.injected && A.sampler == UMAPCU_NEG_REF_HASH && !A.precise_pow;
-    const bool fast5 = fast && A.neg_rate == 5;
-    const unsigned grid = ceil_div(nseg, kWarps);
-    const EpochForm f = epoch_form<D, DENS>(nseg, A.rec != nullptr, fast5);
+    const bool fast5 = fast_config(A);
+    const EpochForm f = epoch_form<D, DENS>(A);
     if (f.warps && A.rec) {
         if (fast5 && f.warps == 3) launch_one(k_epoch_split<D, DENS, 5, true, 3>, nseg, 96, A, f.dependent, s);
         else if (fast5 && f.warps == 6) launch_one(k_epoch_split<D, DENS, 5, true, 6>, nseg, 192, A, f.dependent, s);
         else if (fast5) launch_one(k_epoch_split<D, DENS, 5, true, 4>, nseg, 128, A, f.dependent, s);
         else if (A.neg_rate == 5) launch_one(k_epoch_split<D, DENS, 5, false, 4>, nseg, 128, A, f.dependent, s);
         else launch_one(k_epoch_split<D, DENS, 0, false, 4>, nseg, 128, A, f.dependent, s);
-    } else if (f.warps && A.bits) {
+    } else if (f.warps) {
         if (fast5 && f.warps == 3) launch_one(k_epoch_split_bits<D, DENS, 5, true, 3>, nseg, 96, A, f.dependent, s);
         else if (fast5 && f.warps == 6) launch_one(k_epoch_split_bits<D, DENS, 5, true, 6>, nseg, 192, A, f.dependent, s);
         else if (fast5) launch_one(k_epoch_split_bits<D, DENS, 5, true, 8>, nseg, 256, A, f.dependent, s);
         else if (A.neg_rate == 5) launch_one(k_epoch_split_bits<D, DENS, 5, false, 8>, nseg, 256, A, f.dependent, s);
         else launch_one(k_epoch_split_bits<D, DENS, 0, false, 8>, nseg, 256, A, f.dependent, s);
-    } else if (f.plain() && fast5 && D <= 2 && (A.rec || A.bits)) {
-        if constexpr (D <= 2) {
-            if (A.rec) launch_one(k_epoch<D, DENS, 5, true, true, false, true>, grid, kWarps * 32, A, false, s);
-            else launch_one(k_epoch<D, DENS, 5, true, false, true, true>, grid, kWarps * 32, A, false, s);
+    } else if constexpr (D <= 2) {
+        // (launched after its predecessor with the coherent loads: 60k points, powf
+        // 22.1 -> 23.2 us, four negatives 16.6 -> 17.5; above two dimensions 2 %)
+        if (f.dependent) {
+            if (fast5) launch_warps<D, DENS, 5, true, false>(A, true, s);
+            else if (A.neg_rate == 5) launch_warps<D, DENS, 5, false, false>(A, true, s);
+            else launch_warps<D, DENS, 0, false, false>(A, true, s);
+        } else {
+            if (fast5) launch_warps<D, DENS, 5, true, true>(A, false, s);
+            else if (A.neg_rate == 5) launch_warps<D, DENS, 5, false, true>(A, false, s);
+            else launch_warps<D, DENS, 0, false, true>(A, false, s);
         }
-    } else if (A.rec) {
-        if (fast5) launch_one(k_epoch<D, DENS, 5, true, true>, grid, kWarps * 32, A, f.dependent, s);
-        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5, false, true>, grid, kWarps * 32, A, f.dependent, s);
-        else launch_one(k_epoch<D, DENS, 0, false, true>, grid, kWarps * 32, A, f.dependent, s);
-    } else if (A.bits) {
-        if (fast5) launch_one(k_epoch<D, DENS, 5, true, false, true>, grid, kWarps * 32, A, f.dependent, s);
-        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5, false, false, true>, grid, kWarps * 32, A, f.dependent, s);
-        else launch_one(k_epoch<D, DENS, 0, false, false, true>, grid, kWarps * 32, A, f.dependent, s);
     } else {
-        const uint32_t P = epoch_min_blocks<D, DENS, false>() * kWarps * (uint32_t)device_sm_count();
-        const bool dependent = 2 * nseg <= P || nseg > 2 * P;
-        if (fast5) launch_one(k_epoch<D, DENS, 5, true>, grid, kWarps * 32, A, dependent, s);
-        else if (A.neg_rate == 5) launch_one(k_epoch<D, DENS, 5>, grid, kWarps * 32, A, dependent, s);
-        else launch_one(k_epoch<D, DENS, 0>, grid, kWarps * 32, A, dependent, s);
+        if (fast5) launch_warps<D, DENS, 5, true, false>(A, f.dependent, s);
+        else if (A.neg_rate == 5) launch_warps<D, DENS, 5, false, false>(A, f.dependent, s);
+        else launch_warps<D, DENS, 0, false, false>(A, f.dependent, s);
     }
 }
 
@@ -572,13 +667,9 @@ void launch_epoch(const EpochArgs &A, uint32_t n_dim, bool dens, cudaStream_t s)
     check_launch("k_epoch");
 }
 
-void launch_dens_update(const DensArgs &Dn, uint32_t n_dim, cudaStream_t s)
+void launch_dens_update(const DensArgs &Dn, uint32_t n_dim, bool dependent, cudaStream_t s)
 {
     const uint32_t nb = ceil_div(Dn.n, kDensBlock);
-    // Dependent where the grid fits beside the epoch kernel before it, or is
-    // larger than the device (epoch_form)
-    const uint32_t slots = 8u * (uint32_t)device_sm_count();
-    const bool dependent = 2 * nb <= slots || nb > slots;
 #define UMAPCU_CASE(DD)                                                   \
     case DD:                                                              \
         if (Dn.precise_pow) launch_one(k_dens_update<DD, true>, nb, kDensBlock, Dn, dependent, s); \

@@ -82,7 +82,10 @@ void launch_resident_fits(const uint32_t *offsets, uint32_t n, uint32_t *status,
 size_t resident_ring_bytes(uint32_t n);
 bool launch_layout_resident(const EpochArgs &A, uint32_t n_dim, const float4 *scal, uint32_t first, uint32_t count,
                             uint64_t words, uint4 *ring, uint32_t *counter, uint32_t *status, cudaStream_t s);
-void launch_dens_update(const DensArgs &D, uint32_t n_dim, cudaStream_t s);
+// Whether a density epoch's radii are launched dependent on the kernel before
+// them (A: the epoch's schedule and configuration).
+bool density_radii_dependent(const EpochArgs &A, uint32_t n_dim);
+void launch_dens_update(const DensArgs &D, uint32_t n_dim, bool dependent, cudaStream_t s);
 uint32_t dens_partials(uint32_t n);
 void launch_adam_apply(const float *grad, const uint32_t *hu, float *m, float *v, float *y, uint64_t n_total,
                        uint32_t n_dim, float fused, float epsc, float omb1, float omb2, cudaStream_t s);
