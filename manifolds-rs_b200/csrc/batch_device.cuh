@@ -156,12 +156,16 @@ __global__ void __launch_bounds__(kWarps * 32, 8) k_batch_epoch(const BatchArgs 
 
 // Dependent unless the grid fits the device but not beside the one before it,
 // whose leftovers its blocks would then be packed onto (epoch_form in
-// layout.cu).
+// layout.cu): from half the blocks it holds on, and in the fast configuration,
+// whose blocks are short, from three a SM in two dimensions (564 blocks 14.8 us
+// an epoch, dependent 16.3; 314: 13.0, 11.8), one in three (63: 14.0, 13.2; 252:
+// 18.7, 20.8; 564: 28.0, 35.6) and two in four (252: 14.5, 14.2; 376: 15.9, 16.6).
 template <int D, int NR, int KU, bool FAST, bool BITS>
 inline void launch_batch_epoch(const BatchArgs &B, uint32_t e, cudaStream_t s)
 {
-    const unsigned grid = ceil_div(B.n_segs, kWarps), slots = 8u * (unsigned)device_sm_count();
-    if (2 * grid > slots && grid <= slots) {
+    const unsigned grid = ceil_div(B.n_segs, kWarps), sms = (unsigned)device_sm_count(), slots = 8u * sms;
+    const unsigned beside = !FAST ? slots / 2 : D == 2 ? 3 * sms : D == 3 ? sms : 2 * sms;
+    if (grid > beside && grid <= slots) {
         k_batch_epoch<D, NR, KU, FAST, BITS, false><<<grid, kWarps * 32, 0, s>>>(B, e);
         return;
     }
