@@ -817,11 +817,14 @@ void batched_component_raw(uint32_t n, const DevBuf<uint64_t> &ptr, const DevBuf
     }
     // per component: truncate, tridiagonal eigenproblem; the Ritz coefficients
     // of its kk smallest eigenvalues, c [kk][it_max][S]. On the device for
-    // several components of up to kTridiagRows rows (both matrices in shared
-    // memory); a single one is as fast on the host.
+    // three and more components of up to kTridiagRows rows (both matrices in
+    // shared memory). A single one is as fast on the host, and two are while
+    // they are short: whole calls of 2 x 1000 points in 2 / 8 / 15 dimensions
+    // (42, 66, 94 rows), host and device, 4.9, 5.6; 10.9, 11.8; 23.9, 22.2 ms;
+    // three 5.6, 5.6; 13.3, 12.0.
     std::vector<uint32_t> found(S);
-    constexpr uint32_t kTridiagRows = 110;
-    if (S > 1 && it_max <= kTridiagRows) {
+    constexpr uint32_t kTridiagRows = 110, kTwoRows = 84;
+    if ((S > 2 || (S == 2 && it_max > kTwoRows)) && it_max <= kTridiagRows) {
         auto smem_of = [](uint32_t r) { return 2 * sizeof(double) * r * (r | 1u); };
         const size_t smem = smem_of(it_max);
         // the most of any call: the attribute is the function's, shared by all threads
