@@ -572,6 +572,13 @@ umapcu_status umapcu_dens_state_new(uint32_t n, uint64_t nnz, const uint32_t *ro
         if (!r || !mu_sum || !mu_tot || !knn_idx || !knn_dist || k == 0) return UMAPCU_BAD_ARG;
         if (nnz && (!row || !col || !val)) return UMAPCU_BAD_ARG;
         const uint64_t nk = (uint64_t)n * k;
+        // the indices are checked before anything reads at their places (a
+        // negative neighbour is one past any n)
+        const uint32_t limit = std::min(n, 1u << 31);
+        const bool on_host = 2 * nnz + nk <= kHostCheck;
+        if (on_host && !(in_range(row, nnz, n, true) && in_range(col, nnz, n, false) &&
+                         in_range((const uint32_t *)knn_idx, nk, limit, false)))
+            return UMAPCU_BAD_ARG;
         Stream S;
         DevBuf<uint32_t> dr(nnz, S.s), dc(nnz, S.s), bad(1, S.s);
         DevBuf<float> dv(nnz, S.s), dd(nk, S.s), outr(n, S.s), outm(n, S.s);
@@ -579,18 +586,20 @@ umapcu_status umapcu_dens_state_new(uint32_t n, uint64_t nnz, const uint32_t *ro
         h2d(dr.p, row, nnz, S.s);
         h2d(dc.p, col, nnz, S.s);
         h2d(di.p, knn_idx, nk, S.s);
-        // the indices are checked before anything reads at their places (a
-        // negative neighbour is one past any n)
-        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), S.s), "memset");
-        check_range_dev(dr.p, nnz, n, true, bad.p, S.s);
-        check_range_dev(dc.p, nnz, n, false, bad.p, S.s);
-        check_range_dev((const uint32_t *)di.p, nk, std::min(n, 1u << 31), false, bad.p, S.s);
+        if (!on_host) {
+            check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), S.s), "memset");
+            check_range_dev(dr.p, nnz, n, true, bad.p, S.s);
+            check_range_dev(dc.p, nnz, n, false, bad.p, S.s);
+            check_range_dev((const uint32_t *)di.p, nk, limit, false, bad.p, S.s);
+        }
         h2d(dv.p, val, nnz, S.s);
         h2d(dd.p, knn_dist, nk, S.s);
-        uint32_t bad_h = 0;
-        d2h(&bad_h, bad.p, 1, S.s);
-        sync(S.s);
-        if (bad_h) return UMAPCU_BAD_ARG;
+        if (!on_host) {
+            uint32_t bad_h = 0;
+            d2h(&bad_h, bad.p, 1, S.s);
+            sync(S.s);
+            if (bad_h) return UMAPCU_BAD_ARG;
+        }
         umapcu_status rc =
             dens_state_dev(n, nnz, dr.p, dc.p, dv.p, di.p, dd.p, k, distances_squared, outr.p, outm.p, mu_tot, S.s);
         if (rc != UMAPCU_OK) return rc;

@@ -180,8 +180,19 @@ void construct_graph_dev(const int32_t *d_idx, const float *d_dist, uint32_t n, 
                          const umapcu_graph_params &gp, uint32_t n_epochs, DeviceCoo &out,
                          float *d_sigma, float *d_rho, cudaStream_t s);
 
-// Sets *d_bad when one of m indices is outside [0, limit) or, if ascending, below
-// the one before it (graph.cu).
+// Index checks of the callers' arrays: on the host up to kHostCheck entries in all
+// (0.5 ns an entry; the device's launches, copy back and wait take some 15 us),
+// else on the device once they are there.
+constexpr uint64_t kHostCheck = 32768;
+// Whether all of m indices are below limit and, if ascending, none below the one
+// before it.
+inline bool in_range(const uint32_t *v, uint64_t m, uint32_t limit, bool ascending)
+{
+    bool ok = true;
+    for (uint64_t i = 0; i < m; i++) ok = ok && v[i] < limit && !(ascending && i && v[i] < v[i - 1]);
+    return ok;
+}
+// Sets *d_bad when one is not (graph.cu).
 void check_range_dev(const uint32_t *d_v, uint64_t m, uint32_t limit, bool ascending, uint32_t *d_bad, cudaStream_t s);
 
 // densMAP constant state (density.rs:181-201) on device buffers.

@@ -756,6 +756,8 @@ umapcu_status umapcu_fuzzy_cross_entropy(const uint32_t *row, const uint32_t *co
             *out = 0.0;
             return UMAPCU_OK;
         }
+        const bool on_host = 2 * nnz <= kHostCheck;
+        if (on_host && !(in_range(row, nnz, n, false) && in_range(col, nnz, n, false))) return UMAPCU_BAD_ARG;
         keep_pool_memory();
         Stream st;
         cudaStream_t s = st.s;
@@ -764,15 +766,19 @@ umapcu_status umapcu_fuzzy_cross_entropy(const uint32_t *row, const uint32_t *co
         h2d(dr.p, row, nnz, s);
         h2d(dc.p, col, nnz, s);
         DevBuf<uint32_t> bad(1, s);
-        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
-        check_range_dev(dr.p, nnz, n, false, bad.p, s);
-        check_range_dev(dc.p, nnz, n, false, bad.p, s);
+        if (!on_host) {
+            check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), s), "memset");
+            check_range_dev(dr.p, nnz, n, false, bad.p, s);
+            check_range_dev(dc.p, nnz, n, false, bad.p, s);
+        }
         h2d(dw.p, w, nnz, s);
         h2d(dy.p, y, (size_t)n * n_dim, s);
-        uint32_t bad_h = 0;
-        d2h(&bad_h, bad.p, 1, s);
-        sync(s);
-        if (bad_h) return UMAPCU_BAD_ARG;
+        if (!on_host) {
+            uint32_t bad_h = 0;
+            d2h(&bad_h, bad.p, 1, s);
+            sync(s);
+            if (bad_h) return UMAPCU_BAD_ARG;
+        }
         *out = 0.0;
         const unsigned blocks = ceil_div(nnz, 256);
         DevBuf<double> part(blocks, s);

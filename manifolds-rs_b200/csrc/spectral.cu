@@ -973,6 +973,8 @@ umapcu_status umapcu_spectral_layout(const uint32_t *row, const uint32_t *col, c
     return guard_s([&]() -> umapcu_status {
         if (n == 0) return UMAPCU_NO_DATA;
         if (!embd || n_comp == 0 || n_comp > 64 || (nnz && (!row || !col || !val))) return UMAPCU_BAD_ARG;
+        const bool on_host = 2 * nnz <= kHostCheck;
+        if (on_host && !(in_range(row, nnz, n, false) && in_range(col, nnz, n, false))) return UMAPCU_BAD_ARG;
         const double rng = range > 0.0f ? (double)range : 10.0;  // SPECTRAL_RANGE, init.rs:17
         keep_pool_memory();
         Stream st;
@@ -993,14 +995,16 @@ umapcu_status umapcu_spectral_layout(const uint32_t *row, const uint32_t *col, c
         DevBuf<uint32_t> drow(nnz ? nnz : 1, st.s), dcol(nnz ? nnz : 1, st.s);
         h2d(drow.p, row, nnz, st.s);
         h2d(dcol.p, col, nnz, st.s);
-        DevBuf<uint32_t> bad(1, st.s);
-        check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), st.s), "memset");
-        check_range_dev(drow.p, nnz, n, false, bad.p, st.s);
-        check_range_dev(dcol.p, nnz, n, false, bad.p, st.s);
-        uint32_t bad_h = 0;
-        d2h(&bad_h, bad.p, 1, st.s);
-        sync(st.s);
-        if (bad_h) return UMAPCU_BAD_ARG;
+        if (!on_host) {
+            DevBuf<uint32_t> bad(1, st.s);
+            check_cuda(cudaMemsetAsync(bad.p, 0, sizeof(uint32_t), st.s), "memset");
+            check_range_dev(drow.p, nnz, n, false, bad.p, st.s);
+            check_range_dev(dcol.p, nnz, n, false, bad.p, st.s);
+            uint32_t bad_h = 0;
+            d2h(&bad_h, bad.p, 1, st.s);
+            sync(st.s);
+            if (bad_h) return UMAPCU_BAD_ARG;
+        }
         component_labels(n, nnz, drow, dcol, root, st.s);
         lap("components");
         std::vector<uint32_t> cid(n, ~0u);
