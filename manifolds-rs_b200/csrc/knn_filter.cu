@@ -1089,23 +1089,27 @@ uint32_t rank_stages(uint32_t chunks, uint32_t k)
 // kernel of few queries keeps its SMs busy the longer, the filter's few blocks
 // do not), but from 160 + n / 4000 on. (The preparation of n points and the
 // tile kernel's work per query are both linear in n; a longer list costs the
-// tile kernel more.) Below kFilterPoints points the sample is too small for
+// tile kernel more, and lists of one or two so little that it keeps several times
+// the queries and pairs.) Below kFilterPoints points the sample is too small for
 // its groups, and beyond 191 dims the operands no longer fit beside the ring.
 // us, k_knn_tile and the filter, queries chosen from n points on the device:
 //   10k x 50, k = 3     256 queries 134, 180   1000 178, 189    2000 265, 205
 //   100k x 190, k = 15  256 980, 1241          1000 2430, 1247
 //   1M x 50, k = 3      64 633, 1777           256 1689, 1751   512 3099, 1816
+// relative to the tile kernel, 2 dims, k = 1: 2600 points 0.77, 4000 0.95, 7000
+// 1.46, 2000 queries of 12 000 1.00, of 50 000 1.28; k = 2: 2600 0.99, 4000 1.23;
 // and whole calls over all points, k = 15: 2048 points x 2 / 50 / 190 dims 472,
 // 306; 514, 354; 628, 569; 4096 points 646, 338; 753, 435; 1120, 786.
 bool knn_filter_takes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k)
 {
     constexpr uint32_t kFilterPoints = 2048;
     constexpr uint64_t kFilterPairs = 4u << 20;
-    if (n < kFilterPoints || n >= (1u << 30) || (uint64_t)n * nq < kFilterPairs || k + 1 >= kGroups) return false;
+    const uint64_t pairs = kFilterPairs * (k < 3 ? 4 - k : 1);
+    if (n < kFilterPoints || n >= (1u << 30) || (uint64_t)n * nq < pairs || k + 1 >= kGroups) return false;
     if (dim > 3u * kChunkK || pack_of(dim).chunks > kMaxChunks) return false;
-    const double few = (500.0 + 10.0 * dim) * std::min(1.0, std::sqrt(12000.0 / n));
-    const double least = std::sqrt(3.0 / k) * std::max(std::min(512.0, 160.0 + n / 4000.0), few);
-    return nq >= least;
+    const double list = std::sqrt(3.0 / k);
+    const double few = k == 1 ? 2600.0 + 10.0 * dim : k == 2 ? 1000.0 + 10.0 * dim : list * (500.0 + 10.0 * dim);
+    return nq >= few * std::min(1.0, std::sqrt(12000.0 / n)) && nq >= list * std::min(512.0, 160.0 + n / 4000.0);
 }
 
 bool knn_filter(const KnnFilterArgs &A, uint32_t *left, uint32_t *n_left, cudaStream_t s)

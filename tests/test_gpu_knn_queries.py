@@ -25,11 +25,14 @@ def _chosen(X, q, k, metric):
 
 
 # the line between the two: 6000 x 10, k = 3: 600 (below it 4M pairs: 700);
-# 6000 x 190, k = 15: 1074; 50k x 20, k = 3: 343; 300k x 4, k = 32: 72
+# 6000 x 190, k = 15: 1074; 50k x 20, k = 3: 343; 300k x 4, k = 32: 72; 6000 x 10,
+# k = 1: 2700 (12M pairs: 2098), k = 2: 1399 (8M); 20k x 4, k = 1: 2045
 @pytest.mark.parametrize("n,dim,k,metric,counts", [(6000, 10, 3, "euclidean", (1, 64, 65, 699, 700, 2000)),
                                                    (6000, 190, 15, "cosine", (129, 1073, 1075)),
                                                    (50_000, 20, 3, "euclidean", (5, 342, 344, 513)),
-                                                   (300_000, 4, 32, "euclidean", (63, 71, 73, 200))])
+                                                   (300_000, 4, 32, "euclidean", (63, 71, 73, 200)),
+                                                   (6000, 10, 1, "euclidean", (2699, 2700)), (6000, 10, 2, "cosine", (1398, 1399)),
+                                                   (20_000, 4, 1, "euclidean", (2044, 2046))])
 def test_chosen_queries(n, dim, k, metric, counts):
     rng = np.random.default_rng(n + dim)
     X = (rng.normal(size=(n, dim)) * rng.uniform(0.3, 2, (n, 1))).astype(np.float32)
